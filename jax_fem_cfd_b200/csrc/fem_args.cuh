@@ -6,15 +6,14 @@
 #include "fem_conv3.cuh"
 
 #define FEM_THREADS 512
+#define FEM_CG_THREADS 256  // 2D k_cg / k_vcycle
 #define FEM_OP_THREADS 256
-// whole dynamic smem of k_cg / k_vcycle: reduction scratch + tile staging + stencil tables
-#define FEM_DYN_SMEM_MAX ((128 + FEM_TILE_SMEM + FEM_TAB_SMEM + FEM_BLK_SMEM) * 8)
-// coarse multigrid levels: at most FEM_MG_TEAM CTAs, levels of at most
-// FEM_MG_TEAM_NN nodes (both can be overridden by the environment variables of
-// the same names)
-#define FEM_MG_TEAM 16
-#define FEM_MG_TEAM_NN 4096
-
+// dynamic smem of k_cg / k_vcycle (doubles): reduction scratch, tile staging, the
+// levels' tables; at most 14 levels of 16 classes x 25 coefficients twice
+#define FEM_CG_SMEM (128 + FEM_TILE_SMEM)
+static_assert(FEM_CG_THREADS * FEM_RING_SLOTS <= FEM_TILE_SMEM, "the strips' rings fit the tile region");
+static_assert(FEM_THREADS * FEM_RING_SLOTS <= FEM_CONV_SMEM, "and the packed kernel's");
+#define FEM_DYN_SMEM_MAX ((FEM_CG_SMEM + FEM_MAX_LEVELS * (2 * 400 + 2 * 16)) * 8)
 struct BiArgs {
   FemSync sync;
   FemGrid g;
@@ -180,13 +179,42 @@ int mixmom_solve(MixMom* M, const FemQuadTab& qt, const double* fq64, const doub
                  const uint8_t* mask, const double* b, double* x, double tol, int inner, int max_cycles,
                  int* cycles, int* status, int sms, cudaStream_t s, cudaStream_t cs);
 
+// In-place Gauss-Jordan inverse of the n x n SPD matrix A on stream s (k_mg3.cu;
+// gj: 2 n doubles of scratch; returns after the work is done)
+int fem_gj_invert(double* A, double* gj, int n, int cap, cudaStream_t s);
+// A (n x n, zeroed by the call): the 2D level's Laplacian from its stencil table,
+// rows and columns of pin replaced by the identity's
+int fem_launch_dense_rows(const FemGrid& g, const double* tab, const uint8_t* pin, double* A, int cap, cudaStream_t s);
+
+// Dense operators of the coarse multigrid levels (k_dense.cu): level l's V-cycle
+// as one n x n matrix, for the coarsest levels of at most FEM_DENSE_NN nodes.
+#define FEM_DENSE_NN 1700
+// mg_dense applies the finest level whose matrix is at most this many entries
+// per CTA
+#define FEM_DENSE_ENTRIES 36000
+struct FemDenseLevel {
+  FemGrid g;
+  FemLattice lat;
+  const double *tab, *tab_off, *invD;  // invD: 1 / diag, 0 on gamma_p (pinned)
+  const uint8_t* pin;                  // pinned mode, else null
+};
+struct FemDense;  // shared by the contexts whose coarse levels are the same
+// The matrices of lv[0..nlev) (finest first; the whole hierarchy from some level
+// down), from the registry or built on stream s; *out owns a reference. FEM_OK
+// with *out null where no level qualifies.
+int fem_dense_acquire(FemDense** out, const FemDenseLevel* lv, int nlev, int pinned, double lx, double ly, int device,
+                      int sms, cudaStream_t s);
+void fem_dense_release(FemDense* d);
+// matrix and row pitch of the level with `from_end` levels below it, null if none
+const double* fem_dense_matrix(const FemDense* d, int from_end, int* ld);
+
 int fem_coop_occupancy_cg(int* occ);
 int fem_coop_occupancy_bi(int* occ);
 int fem_launch_cg(const CgArgs& A, int grid, double* cr, double* cp, double* cq, cudaStream_t s);
 int fem_launch_vcycle(const CgArgs& A, int grid, double* cr, double* cp, double* cq, double* z, cudaStream_t s);
 int fem_launch_bicgstab(int ncomp, const BiArgs& A, int grid, cudaStream_t s);
 // packed step (k_pack.cu): k members of `ctas` CTAs each, one cooperative launch
-int fem_launch_step_pack(int kind, const PackMember* members, const PackParams& P, int k, int ctas, int blk,
+int fem_launch_step_pack(int kind, int periodic, const PackMember* members, const PackParams& P, int k, int ctas,
                          cudaStream_t s);
 int fem_pack_occupancy(int* per_sm);
 

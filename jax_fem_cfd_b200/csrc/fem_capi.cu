@@ -121,9 +121,11 @@ struct fem_ctx {
   uint8_t *dmask = nullptr, *pmask = nullptr, *aipin = nullptr;
   int has_dmask = 0, set_zeroP = 1;
   // multigrid
-  int nlev = 0, block_from = 0;
+  int nlev = 0;
   double coarse_tol = 1e-8;
   CtxLevel lv[FEM_MAX_LEVELS];
+  FemDense* dense = nullptr;      // dense operators of the coarse levels (2D), shared between contexts
+  const uint8_t* pin0 = nullptr;  // the gamma_p mask that level 0's winvD was made from
   double *cr = nullptr, *cp = nullptr, *cq = nullptr;  // coarse CG scratch
   // barrier / reduction state
   unsigned int* bar = nullptr;
@@ -132,7 +134,7 @@ struct fem_ctx {
   int max_coop = 148;       // CTAs of the persistent cooperative launches
   int coop_capacity = 148;  // upper bound of max_coop (co-resident capacity)
   // vectors (nn or ndim*nn)
-  double *pr = nullptr, *pz = nullptr, *pp0 = nullptr, *pp1 = nullptr, *pAp = nullptr, *pb = nullptr;  // CG
+  double *pr = nullptr, *pz = nullptr, *pp0 = nullptr, *pp1 = nullptr, *pAp = nullptr;  // CG
   double *br = nullptr, *brh = nullptr, *bp0 = nullptr, *bp1 = nullptr, *bq0 = nullptr, *bq1 = nullptr,
          *bt = nullptr;                                                                      // BiCGSTAB
   double *rhsU = nullptr, *Uhat = nullptr, *gPn = nullptr, *Ustar = nullptr, *rhsP = nullptr;  // step
@@ -193,9 +195,50 @@ static int dalloc(T** p, size_t n) {
     if (_r) return _r;                  \
   } while (0)
 
-static int ctx_grid_for(const fem_ctx* c, long long work) {
-  // enough CTAs for ~1 node per thread, capped by co-residency
-  return nblocks(work, FEM_THREADS, c->max_coop);
+// Whether the pressure solve may use the dense coarse operators: always on a
+// mean-zero hierarchy (the same linear map), on a pinned one when the coarsest
+// CG is asked for at least six digits, so that the exact inverse stands for it.
+static bool dense_usable(const fem_ctx* c) { return c->dense && (!c->set_zeroP || c->coarse_tol <= 1e-6); }
+
+// CTAs of the persistent BiCGSTAB and of a packed member: ~1 node per thread, capped
+// by co-residency.
+static int ctx_grid_for(const fem_ctx* c) { return nblocks(c->g.nn, FEM_THREADS, c->max_coop); }
+
+// A CG solve whose bits depend on its work items, not its grid (fem_items)
+static bool cg_by_items(const fem_ctx* c) { return c->g.kind == FEM_Q1_2D && c->set_zeroP; }
+
+// CTAs whose matrix share picks the dense level of a solve by items
+static long long dense_ctas(const fem_ctx* c) { return cg_by_items(c) ? ctx_grid_for(c) : c->max_coop; }
+
+// The level from which a solve applies the dense coarse operator: the finest whose
+// matrix is at most FEM_DENSE_ENTRIES entries per CTA, where its product costs as
+// much as the sweeps it stands for. The coarsest pinned one stands for a whole CG
+// inside one CTA, so it is taken at every size.
+static int dense_level(const fem_ctx* c, const double** C, int* ld) {
+  if (dense_usable(c))
+    for (int l = 0; l < c->nlev; ++l) {
+      const long long n = c->lv[l].g.nn;
+      *C = fem_dense_matrix(c->dense, c->nlev - 1 - l, ld);
+      if (*C && (n * n <= dense_ctas(c) * FEM_DENSE_ENTRIES || (c->set_zeroP && l == c->nlev - 1))) return l;
+    }
+  return c->nlev;
+}
+
+// Work items of a 2D CG solve (strip plans, chunks, partial columns): those of
+// ctx_grid_for CTAs of 16 warps, at most one round of the whole device.
+static int cg_items(const fem_ctx* c) { return std::min(ctx_grid_for(c) * 16, c->sms * (FEM_CG_THREADS / 32)); }
+
+// CTAs of a CG solve. 2D: one warp of work per CTA while there are items (a warp
+// alone on its SM runs fastest: 64^2 quad4 cavity step on 9 CTAs 541 us, on 145
+// 373 us), and enough for the dense level's rows.
+static int cg_grid_for(const fem_ctx* c) {
+  if (c->g.kind == FEM_HEX8) return ctx_grid_for(c);
+  if (cg_by_items(c)) return std::min(cg_items(c), c->max_coop);
+  const double* C;
+  int ld;
+  const int d = dense_level(c, &C, &ld);
+  const long long n = d < c->nlev ? c->lv[d].g.nn : 0;
+  return std::max(nblocks(c->g.nn, 64, c->max_coop), nblocks((n + 7) / 8, 1, c->max_coop));
 }
 
 // --------------------------------------------------------------- mesh ----
@@ -290,9 +333,10 @@ extern "C" void fem_ctx_destroy(fem_ctx* c) {
   mg3_destroy(c->mg3);
   mg3_destroy(c->mg2);
   mixmom_destroy(c->mixmom);
+  fem_dense_release(c->dense);
   void* ptrs[] = {c->coords, c->wq, c->N, c->dN, c->Me, c->Le, c->Leoff, c->Ge, c->M, c->Ldiag, c->Kd,
                   c->dmask, c->pmask, c->aipin, c->cr, c->cp, c->cq, c->bar, c->err, c->partials, c->pr,
-                  c->pz, c->pp0, c->pp1, c->pAp, c->pb, c->br, c->brh, c->bp0, c->bp1, c->bq0, c->bq1, c->bt,
+                  c->pz, c->pp0, c->pp1, c->pAp, c->br, c->brh, c->bp0, c->bp1, c->bq0, c->bq1, c->bt,
                   c->rhsU, c->Uhat, c->gPn, c->Ustar, c->rhsP, c->Ce, c->Ce2, c->Ct, c->Mt, c->Ek, c->tau,
                   c->dotpart, c->Fe, c->flags, c->vcv, c->cvf, c->ebe_tab, c->bs_cnt, c->bs_off, c->bs_list, c->vjp, c->vjp2,
                   c->step_tab};
@@ -420,13 +464,13 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   FEM_ALLOC(c->M, vn);
   FEM_ALLOC(c->Ldiag, nn);
   FEM_ALLOC(c->dmask, vn);
-  FEM_ALLOC(c->pmask, nn);
-  FEM_ALLOC(c->aipin, nn);
-  FEM_ALLOC(c->bar, 2);
+  FEM_ALLOC(c->pmask, nn + 4);  // whole words (fem_ring_copy_mask)
+  FEM_ALLOC(c->aipin, nn + 4);
+  FEM_ALLOC(c->bar, 1);
   FEM_ALLOC(c->err, 1);
-  FEM_ALLOC(c->partials, (size_t)FEM_NSLOTS * c->max_coop);
+  FEM_ALLOC(c->partials, (size_t)FEM_NSLOTS * std::max(c->max_coop, c->sms * (FEM_CG_THREADS / 32)));
   FEM_ALLOC(c->flags, 16);
-  for (double** p : {&c->pr, &c->pz, &c->pp0, &c->pp1, &c->pAp, &c->pb, &c->rhsP}) FEM_ALLOC(*p, nn);
+  for (double** p : {&c->pr, &c->pz, &c->pp0, &c->pp1, &c->pAp, &c->rhsP}) FEM_ALLOC(*p, nn);
   for (double** p : {&c->br, &c->brh, &c->bp0, &c->bp1, &c->bq0, &c->bq1, &c->bt, &c->rhsU, &c->Uhat, &c->gPn,
                      &c->Ustar})
     FEM_ALLOC(*p, vn);
@@ -436,7 +480,7 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   FEM_ALLOC(c->cvf, g.kind == FEM_HEX8 ? (size_t)FEM_C3_NF * g.ne : (size_t)3 * c->nq * g.ne);
   FEM_ALLOC(c->dotpart, 4096);
   cudaStream_t s = 0;
-  FEM_CHECK(cudaMemset(c->bar, 0, 2 * sizeof(unsigned int)));
+  FEM_CHECK(cudaMemset(c->bar, 0, sizeof(unsigned int)));
   FEM_CHECK(cudaMemset(c->err, 0, sizeof(int)));
   FEM_CHECK(cudaMemset(c->flags, 0, 16 * sizeof(int)));
   FEM_CHECK(cudaMemset(c->dmask, 0, vn));
@@ -551,6 +595,26 @@ extern "C" int fem_ctx_element_data(const fem_ctx* c, double* wq, double* N, dou
   return FEM_OK;
 }
 
+// The dense coarse operators of the current hierarchy and pressure mode (2D).
+// A context without them (no level small enough, no memory for them) solves its
+// coarsest level in CTA 0.
+static int dense_refresh(fem_ctx* c, cudaStream_t s) {
+  if (c->g.kind == FEM_HEX8 || c->nlev < 2) return FEM_OK;
+  FemDenseLevel lv[FEM_MAX_LEVELS];
+  for (int l = 0; l < c->nlev; ++l) {
+    const CtxLevel& L = c->lv[l];
+    lv[l] = FemDenseLevel{L.g, lattice_of(L.g), L.tab, L.tab_off, c->set_zeroP ? L.winvD : L.invD,
+                          l == 0 ? c->pin0 : L.pin};
+  }
+  FemDense* d = nullptr;
+  const int rc = fem_dense_acquire(&d, lv, c->nlev, c->set_zeroP, c->lx, c->ly, c->device, c->sms, s);
+  if (rc == FEM_E_CUDA && cudaGetLastError() == cudaErrorMemoryAllocation) d = nullptr;
+  else if (rc) return rc;
+  fem_dense_release(c->dense);
+  c->dense = d;
+  return FEM_OK;
+}
+
 extern "C" int fem_ctx_set_bc(fem_ctx* c, const uint8_t* dmask, const uint8_t* pmask, int set_zeroP,
                               cudaStream_t s) {
   if (!c) return FEM_E_ARG;
@@ -566,6 +630,7 @@ extern "C" int fem_ctx_set_bc(fem_ctx* c, const uint8_t* dmask, const uint8_t* p
     FEM_CHECK(cudaMemcpyAsync(c->pmask, pmask, nn, cudaMemcpyDeviceToDevice, s));
     FEM_CHECK(cudaMemcpyAsync(c->aipin, pmask, nn, cudaMemcpyDeviceToDevice, s));
   }
+  const bool mode_changed = c->set_zeroP != (set_zeroP ? 1 : 0);
   c->set_zeroP = set_zeroP ? 1 : 0;
   if (c->mg2) {  // its pins and mean-zero form follow the boundary sets
     FEM_CHECK(cudaStreamSynchronize(s));
@@ -573,6 +638,8 @@ extern "C" int fem_ctx_set_bc(fem_ctx* c, const uint8_t* dmask, const uint8_t* p
     c->mg2 = nullptr;
   }
   FEM_TRY(fem_launch_invdiag(c->g.nn, c->Ldiag, c->pmask, c->lv[0].invD, c->lv[0].winvD, s));
+  c->pin0 = c->pmask;
+  if (c->nlev > 1 && (mode_changed || pmask)) FEM_TRY(dense_refresh(c, s));
   return FEM_OK;
 }
 
@@ -607,6 +674,8 @@ extern "C" int fem_ctx_setup_multigrid(fem_ctx* c, int nlev, const uint8_t* leve
   }
   mg3_destroy(c->mg2);
   c->mg2 = nullptr;
+  fem_dense_release(c->dense);
+  c->dense = nullptr;
   const FemGrid& g0 = c->g;
   for (int l = 1; l < nlev; ++l)
     if ((g0.nex >> l) < 1 || (g0.ney >> l) < 1) return FEM_E_ARG;
@@ -658,7 +727,7 @@ extern "C" int fem_ctx_setup_multigrid(fem_ctx* c, int nlev, const uint8_t* leve
       cudaFree(Mtmp);
       if (rc) break;
     }
-    rc |= dalloc(&L.pin, nn);
+    rc |= dalloc(&L.pin, nn + 4);  // whole words (fem_ring_copy_mask)
     if (rc) break;
     if (level_pmasks) {
       FEM_CHECK(cudaMemcpyAsync(L.pin, level_pmasks + off, nn, cudaMemcpyDeviceToDevice, s));
@@ -706,14 +775,8 @@ extern "C" int fem_ctx_setup_multigrid(fem_ctx* c, int nlev, const uint8_t* leve
   FEM_ALLOC(c->cr, ncn);
   FEM_ALLOC(c->cp, ncn);
   FEM_ALLOC(c->cq, ncn);
-  // First level handled by the coarse-level team: the coarsest levels of at
-  // most FEM_MG_TEAM_NN nodes.
-  int small = FEM_MG_TEAM_NN;
-  if (const char* ev = getenv("FEM_MG_TEAM_NN")) small = atoi(ev);
-  int bf = nlev - 1;
-  for (int l = nlev - 2; l >= 0 && c->lv[l].g.nn <= small; --l) bf = l;
-  c->block_from = bf;
-  return FEM_OK;
+  c->pin0 = c->lv[0].pin;
+  return dense_refresh(c, s);
 }
 
 extern "C" int fem_ctx_level_info(const fem_ctx* c, int level, int* nn, int* nnx, int* nny, int* nex, int* ney) {
@@ -824,38 +887,10 @@ extern "C" int fem_lattice_restrict(int nhx, int nhy, int nHx, int nHy, int peri
   return fem_launch_restrict(FemLattice{nhx, nhy, periodic ? 1 : 0}, FemLattice{nHx, nHy, periodic ? 1 : 0}, xh, xH, s);
 }
 
-// First multigrid level of the V-cycle run inside CTA 0 from shared memory
-// (mg_block_levels): the coarsest levels, from the team's first level down,
-// whose r and x plus one scratch of the finest of them fit the tile region
-// after the warp CG's buffer and whose 1/D fit FEM_BLK_SMEM; pinned pressure
-// also needs a coarsest level the warp CG takes. c->nlev: none. 2D only, and
-// only with FEM_MG_BLOCK=1: on the Taylor-Green 256^2 Q2 solve the CTA-0
-// levels took 36.6 us per V-cycle against ~40 us on the team, and the step
-// ran 470 against 504 steps/s with them.
-static int mg_block_from(const fem_ctx* c) {
-  const int N = c->nlev;
-  if (N < 2 || c->g.kind == FEM_HEX8) return N;
-  const char* ev = getenv("FEM_MG_BLOCK");
-  if (!ev || atoi(ev) != 1) return N;
-  if (c->set_zeroP && c->lv[N - 1].g.nn > FEM_COARSE_WARP_NN) return N;
-  int b = N;
-  long long vec = 0, d = 0;
-  for (int l = N - 1; l >= 1 && l >= c->block_from; --l) {
-    const CtxLevel& L = c->lv[l];
-    if (!L.invD || !L.winvD || !L.r || !L.t) break;
-    vec += 2LL * L.g.nn;
-    d += L.g.nn;
-    if (FEM_COARSE_WARP_NN + vec + L.g.nn > FEM_TILE_SMEM || d > FEM_BLK_SMEM) break;
-    b = l;
-  }
-  return b;
-}
-
 static void fill_cg_args(fem_ctx* c, CgArgs& A) {
   memset(&A, 0, sizeof(A));
-  A.sync = FemSync{c->bar, c->bar + 1, c->err, c->partials, FEM_NSLOTS, c->trace, c->trace_cap};
-  A.nlev = c->nlev;
-  A.block_from = c->block_from;
+  A.sync = FemSync{c->bar, c->err, c->partials, 1, FEM_NSLOTS, c->trace, c->trace_cap};
+  A.nlev = c->g.kind == FEM_HEX8 ? 1 : c->nlev;  // the hex8 hierarchy is k_mg3.cu's
   A.pinned = c->set_zeroP;
   A.coarse_maxiter = 1000;
   A.coarse_tol = c->coarse_tol;
@@ -864,9 +899,8 @@ static void fill_cg_args(fem_ctx* c, CgArgs& A) {
   A.p0 = c->pp0;
   A.p1 = c->pp1;
   A.Ap = c->pAp;
-  A.bwork = c->pb;
   A.ai_pin = c->aipin;
-  for (int l = 0; l < c->nlev; ++l) {
+  for (int l = 0; l < A.nlev; ++l) {
     CtxLevel& L = c->lv[l];
     MgLevel& M = A.lv[l];
     M.g = L.g;
@@ -886,21 +920,35 @@ static void fill_cg_args(fem_ctx* c, CgArgs& A) {
     M.r = (l == 0) ? c->pr : L.r;
     M.t = L.t;
   }
+  for (int l = 0; l < A.nlev; ++l) A.lv[l].mpin = (l == 0 && c->pin0) ? c->pin0 : A.lv[l].pin;
   // level 0 pins of the plain (non-multigrid) solve are the context gamma_p
   if (c->nlev == 1 || !c->lv[0].pin) A.lv[0].pin = c->pmask;
-  A.block_smem_from = mg_block_from(c);
+  A.dense_lv = A.nlev;
 }
 
-// CTAs of the coarse-level multigrid team for a launch of `grid` CTAs
-static int team_size(int grid) {
-  int t = FEM_MG_TEAM;
-  if (const char* ev = getenv("FEM_MG_TEAM")) t = atoi(ev);
-  if (t < 1) t = 1;
-  return t < grid ? t : grid;
+// Plans of a 2D solve: strips of the levels, partial columns, dense level
+static void set_cg_plan(const fem_ctx* c, CgArgs& A) {
+  if (c->g.kind == FEM_HEX8) return;
+  const bool by_items = cg_by_items(c);
+  const int grid = cg_grid_for(c), items = by_items ? cg_items(c) : grid * (FEM_CG_THREADS / 32);
+  A.sync.ncols = by_items ? items : grid;
+  for (int l = 0; l < A.nlev; ++l) {
+    MgLevel& M = A.lv[l];
+    const bool q2 = M.g.kind == FEM_Q2_2D;
+    // quad9: whole row pairs
+    M.pl = fem_strip_plan(M.g.nnx, q2 ? KS<FEM_Q2_2D>::OWN : KS<FEM_Q1_2D>::OWN, M.g.nny, items, q2 ? 2 : 1);
+    if (l + 1 < A.nlev)
+      M.pd = fem_strip_plan(A.lv[l + 1].g.nnx, q2 ? KS<FEM_Q2_2D>::COARSE : KS<FEM_Q1_2D>::COARSE,
+                            A.lv[l + 1].g.nny, items, 1);
+  }
+  A.dense_lv = dense_level(c, &A.dense_C, &A.dense_ld);
+  // mg_dense leaves a sum per block of 8 rows
+  if (by_items && A.dense_lv < A.nlev)
+    A.sync.ncols = std::max(items, (A.lv[A.dense_lv].g.nn + 7) / 8);
 }
 
 static int reset_sync(fem_ctx* c, cudaStream_t s) {
-  FEM_CHECK(cudaMemsetAsync(c->bar, 0, 2 * sizeof(unsigned int), s));  // grid and team arrival counts
+  FEM_CHECK(cudaMemsetAsync(c->bar, 0, sizeof(unsigned int), s));  // the grid barrier's arrival count
   FEM_CHECK(cudaMemsetAsync(c->err, 0, sizeof(int), s));
   return FEM_OK;
 }
@@ -921,8 +969,9 @@ static int run_cg(fem_ctx* c, const double* b, double* x, double tol, double ato
   A.status = status;
   A.final_rr = nullptr;
   FEM_TRY(reset_sync(c, s));
-  const int grid = ctx_grid_for(c, c->g.nn);
-  A.team = team_size(grid);
+  const int grid = cg_grid_for(c);
+  A.sync.ncols = grid;
+  set_cg_plan(c, A);
   double* cr = c->cr ? c->cr : c->pz;
   double* cp = c->cp ? c->cp : c->pz;
   double* cq = c->cq ? c->cq : c->pz;
@@ -999,9 +1048,9 @@ extern "C" int fem_mg_vcycle(fem_ctx* c, const double* r, double* z, cudaStream_
   fill_cg_args(c, A);
   FEM_CHECK(cudaMemcpyAsync(c->pr, r, sizeof(double) * c->g.nn, cudaMemcpyDeviceToDevice, s));
   FEM_TRY(reset_sync(c, s));
-  const int grid = ctx_grid_for(c, c->g.nn);
-  A.team = team_size(grid);
-  return fem_launch_vcycle(A, grid, c->cr, c->cp, c->cq, z, s);
+  set_cg_plan(c, A);
+  A.dense_lv = A.nlev;  // the reference's coarsest solve
+  return fem_launch_vcycle(A, cg_grid_for(c), c->cr, c->cp, c->cq, z, s);
 }
 
 static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t* mask, const double* b, double* x,
@@ -1010,7 +1059,7 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
   if (ncomp < 1 || ncomp > c->ndim) return FEM_E_ARG;  // workspace holds ndim*nn per vector
   BiArgs A;
   memset(&A, 0, sizeof(A));
-  A.sync = FemSync{c->bar, c->bar + 1, c->err, c->partials, FEM_NSLOTS, c->trace, c->trace_cap};
+  A.sync = FemSync{c->bar, c->err, c->partials, 1, FEM_NSLOTS, c->trace, c->trace_cap};
   A.g = c->g;
   A.op = op;
   A.mask = mask;
@@ -1032,7 +1081,8 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
   A.cv_coef = cv_coef;
   A.qt = c->qt;
   FEM_TRY(reset_sync(c, s));
-  return fem_launch_bicgstab(ncomp, A, ctx_grid_for(c, c->g.nn), s);
+  A.sync.ncols = ctx_grid_for(c);
+  return fem_launch_bicgstab(ncomp, A, A.sync.ncols, s);
 }
 
 extern "C" int fem_bicgstab_solve(fem_ctx* c, int ncomp, double alpha, const double* Ash, double beta,
@@ -1484,7 +1534,7 @@ extern "C" int fem_pressure_solve_mixed(fem_ctx* c, const double* b, double* x, 
 extern "C" int fem_selftest_barrier_timeout(fem_ctx* c, int* status, cudaStream_t s) {
   if (!c || !status) return FEM_E_ARG;
   FEM_TRY(reset_sync(c, s));
-  const FemSync S{c->bar, c->bar + 1, c->err, c->partials, FEM_NSLOTS, nullptr, 0};
+  const FemSync S{c->bar, c->err, c->partials, 1, FEM_NSLOTS, nullptr, 0};
   return fem_launch_selftest_barrier(S, status, s);
 }
 
@@ -1507,10 +1557,9 @@ extern "C" int fem_ctx_set_max_ctas(fem_ctx* c, int ctas, int* capacity) {
 // ------------------------------------------------------------ packed steps ----
 
 struct fem_pack {
-  int k = 0, ctas = 0, capacity = 0;
-  int blk = 0;                   // the members' multigrid runs its coarsest levels inside CTA 0
+  int k = 0, ctas = 0, capacity = 0, periodic = 0;
   PackMember* dmem = nullptr;    // k members (device)
-  unsigned int* sync = nullptr;  // [2m] grid and [2m + 1] team arrival counts, [2k + m] error word
+  unsigned int* sync = nullptr;  // [m] arrival count, [k + m] error word
 };
 
 extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, double* const* P0,
@@ -1521,7 +1570,7 @@ extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, d
   *out = nullptr;
   const fem_ctx* c0 = ctxs[0];
   if (!c0) return FEM_E_ARG;
-  const int ctas = ctx_grid_for(c0, c0->g.nn);
+  const int ctas = ctx_grid_for(c0);
   for (int m = 0; m < k; ++m) {
     const fem_ctx* c = ctxs[m];
     if (!c || !U0[m] || !P0[m] || !U1[m] || !P1[m]) return FEM_E_ARG;
@@ -1534,7 +1583,7 @@ extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, d
       return FEM_E_STATE;
     }
     if (c->g.nnx != c0->g.nnx || c->g.nny != c0->g.nny || c->g.periodic != c0->g.periodic ||
-        c->device != c0->device || ctx_grid_for(c, c->g.nn) != ctas) {
+        c->device != c0->device || ctx_grid_for(c) != ctas) {
       snprintf(g_err, sizeof(g_err), "fem_pack_create: member %d differs in mesh, device or CTA count", m);
       return FEM_E_STATE;
     }
@@ -1550,18 +1599,19 @@ extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, d
   fem_pack* p = new fem_pack();
   p->k = k;
   p->ctas = ctas;
+  p->periodic = c0->g.periodic;
   p->capacity = capacity;
   std::vector<PackMember> hm(k);
   int rc = dalloc(&p->dmem, (size_t)k);
-  if (!rc) rc = dalloc(&p->sync, (size_t)3 * k);
+  if (!rc) rc = dalloc(&p->sync, (size_t)2 * k);
   const double theta = 0.5, rho = 1.0;
   for (int m = 0; m < k && !rc; ++m) {
     fem_ctx* c = ctxs[m];
     PackMember& M = hm[m];
     memset(&M, 0, sizeof(M));
     int* st = stat + 5 * m;
-    const FemSync sync{p->sync + 2 * m, p->sync + 2 * m + 1, reinterpret_cast<int*>(p->sync + 2 * k + m),
-                       c->partials, FEM_NSLOTS, nullptr, 0};
+    const FemSync sync{p->sync + m, reinterpret_cast<int*>(p->sync + k + m), c->partials, ctas, FEM_NSLOTS,
+                       nullptr, 0};
     // the fem_step4 stage arguments (dt, mu set per launch)
     StepArgs& S = M.S;
     S.g = c->g;
@@ -1615,8 +1665,7 @@ extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, d
     C.iters = st + 1;
     C.status = st + 3;
     C.final_rr = nullptr;
-    C.team = team_size(ctas);
-    if (C.block_smem_from < C.nlev) p->blk = 1;
+    set_cg_plan(c, C);
     M.U[0] = U0[m];
     M.U[1] = U1[m];
     M.P[0] = P0[m];
@@ -1664,8 +1713,8 @@ extern "C" int fem_pack_step(fem_pack* p, const double* dt, const double* mu, co
              active, p->ctas, p->capacity);
     return FEM_E_STATE;
   }
-  FEM_CHECK(cudaMemsetAsync(p->sync, 0, sizeof(unsigned int) * 3 * p->k, s));
-  return fem_launch_step_pack(FEM_Q1_2D, p->dmem, P, active, p->ctas, p->blk, s);
+  FEM_CHECK(cudaMemsetAsync(p->sync, 0, sizeof(unsigned int) * 2 * p->k, s));
+  return fem_launch_step_pack(FEM_Q1_2D, p->periodic, p->dmem, P, active, p->ctas, s);
 }
 
 extern "C" int fem_pack_info(const fem_pack* p, int* k, int* ctas, int* capacity) {

@@ -172,9 +172,9 @@ __device__ __forceinline__ bool fem_watchdog_fired(const int* err) {
 
 struct FemSync {
   unsigned int* count;    // arrivals in the current barrier generation
-  unsigned int* team_count;  // arrivals at the coarse-level team barrier (GridTeam::team)
   int* err;               // sticky error flags (FEM_ERR_*)
-  double* partials;       // [slot][cta] partial sums
+  double* partials;       // [slot][column] partial sums: one column per CTA, or per work item (2D CG)
+  int ncols;              // columns of a slot
   int nslots;
   unsigned long long* trace;  // optional: globaltimer at each barrier exit (CTA 0), trace[0] = count
   int trace_cap;
@@ -304,7 +304,7 @@ struct FemPartials {
     for (int q = 0; q < K; ++q) {
       double t = 0.0;
       for (int w = 0; w < nw; ++w) t += smem[q * 16 + w];
-      s->partials[(size_t)slots[q] * gridDim.x + blockIdx.x] = t;
+      s->partials[(size_t)slots[q] * s->ncols + blockIdx.x] = t;
     }
   }
 };
@@ -352,10 +352,8 @@ __device__ __forceinline__ bool fem_counter_barrier(const FemSync* s, unsigned i
   return s_ok != 0;
 }
 
-// A set of CTAs that synchronise on one arrival counter: every CTA of the
-// launch (grid(): cooperative, all co-resident), or the first n CTAs (team():
-// the coarse multigrid levels, with their own counter). One type for both, so
-// the phase functions are compiled once.
+// The CTAs that synchronise on one arrival counter: every CTA of a cooperative
+// (co-resident) launch, or of one group of a packed launch.
 struct GridTeam {
   const FemSync* s;     // the launch's barrier state (shared-memory copy of the kernel arguments)
   unsigned int* cnt;    // arrival counter (global)
@@ -364,9 +362,6 @@ struct GridTeam {
   unsigned int tag;     // trace tag of its barriers
   __device__ static GridTeam grid(const FemSync* s, unsigned int* round) {
     return GridTeam{s, s->count, round, (int)gridDim.x, 31u};
-  }
-  __device__ static GridTeam team(const FemSync* s, unsigned int* round, int n) {
-    return GridTeam{s, s->team_count, round, n, 30u};
   }
   __device__ __forceinline__ int rank() const { return blockIdx.x * blockDim.x + threadIdx.x; }
   __device__ __forceinline__ int size() const { return n * blockDim.x; }
@@ -424,8 +419,37 @@ struct GridReducer {
     if (threadIdx.x == 0) {
       double* part = s->partials;
 #pragma unroll
-      for (int q = 0; q < K; ++q) part[(size_t)(slot + q) * gridDim.x + blockIdx.x] = v[q];
+      for (int q = 0; q < K; ++q) part[(size_t)(slot + q) * s->ncols + blockIdx.x] = v[q];
     }
+  }
+  // A warp's sums of K values of work item `item` into column `item` (all lanes call
+  // it; published by the team's next sync). Columns no item writes stay zero.
+  template <int K>
+  __device__ __forceinline__ void warp_item(double (&v)[K], const int (&slots)[K], int item) const {
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int q = 0; q < K; ++q) s->partials[(size_t)slots[q] * s->ncols + item] = v[q];
+  }
+  // Sums of the items a warp runs in one phase, K values in v bound for `slots`:
+  // item_sums after each item, finish_items at the phase's end in place of its
+  // barrier. ITEMS: an item's sums go to a column of its own (v restarts), so they
+  // do not depend on the grid; else they stay in v and join the barrier's block sum.
+  template <bool ITEMS, int K>
+  __device__ __forceinline__ void item_sums(double (&v)[K], const int (&slots)[K], int item) const {
+    if (!ITEMS) return;
+    warp_item<K>(v, slots, item);
+#pragma unroll
+    for (int q = 0; q < K; ++q) v[q] = 0.0;
+  }
+  template <bool ITEMS, int K>
+  __device__ __forceinline__ bool finish_items(const GridTeam& tm, double (&v)[K], const int (&slots)[K],
+                                               double* smem) const {
+    if constexpr (ITEMS) return tm.sync();
+    return tm.template reduce_sync<K>(v, slots, smem);
   }
   // One block sum for K values bound for any K slots.
   template <int K>
@@ -434,13 +458,14 @@ struct GridReducer {
     if (threadIdx.x == 0) {
       double* part = s->partials;
 #pragma unroll
-      for (int q = 0; q < K; ++q) part[(size_t)slots[q] * gridDim.x + blockIdx.x] = v[q];
+      for (int q = 0; q < K; ++q) part[(size_t)slots[q] * s->ncols + blockIdx.x] = v[q];
     }
   }
-  // Totals of K <= 8 slots (any slot numbers). Thread c loads CTA c's partial of
-  // every slot (all loads of a thread in flight at once), warps combine theirs
-  // by a fixed shuffle tree, and every thread adds the warp sums in warp order:
-  // the same order, hence the same bits, in every CTA. Uses smem[0, 16*K).
+  // Totals of K <= 8 slots (any slot numbers). Thread c loads column c (and every
+  // data_warps() * 32th after it) of every slot (all loads of a thread in flight at
+  // once), warps combine theirs by a fixed shuffle tree, and every thread adds the
+  // warp sums in warp order: the same order, hence the same bits, in every CTA and
+  // for every block size. Uses smem[0, 16*K).
   // Split in two so that other loads (a phase's staging copies) can be issued
   // between them: result_begin issues this thread's partial loads,
   // result_end combines them (both called by every thread of the CTA).
@@ -449,16 +474,14 @@ struct GridReducer {
     double acc[K];
   };
   __device__ __forceinline__ int data_warps() const {
-    int nwd = (gridDim.x + 31) >> 5;
-    if (nwd > 16) nwd = 16;
-    if (nwd > (int)(blockDim.x >> 5)) nwd = blockDim.x >> 5;
-    return nwd;
+    const int nwd = (s->ncols + 31) >> 5;
+    return nwd < 8 ? nwd : 8;  // the smallest block of a solver has 8 warps
   }
   template <int K>
   __device__ __forceinline__ Pending<K> result_begin(const int (&slots)[K]) const {
     static_assert(K <= 8, "result_slots: at most 8 slots");
     Pending<K> p;
-    const int G = gridDim.x, nwd = data_warps();
+    const int G = s->ncols, nwd = data_warps();
     const double* __restrict__ part = s->partials;
 #pragma unroll
     for (int q = 0; q < K; ++q) p.acc[q] = 0.0;

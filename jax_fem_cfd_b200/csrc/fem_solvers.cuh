@@ -1,7 +1,8 @@
 // Device-resident Krylov solvers: one persistent cooperative launch runs the
 // whole CG / BiCGSTAB loop. Phases are separated by bounded grid barriers
-// (GridTeam::sync); reductions are two-pass and deterministic; the coarse
-// multigrid levels run inside CTA 0 with __syncthreads only (BlockTeam).
+// (GridTeam::sync); reductions are two-pass and deterministic; the coarse end of
+// the V-cycle is one dense product (mg_dense) or, without one, a coarsest solve
+// inside CTA 0 (BlockTeam).
 // Shared-matrix products (L, L_off) use the assembled stencils of
 // fem_stencil.cuh; the element kind is a template parameter.
 //
@@ -13,6 +14,7 @@
 #pragma once
 #include "fem_ops.cuh"
 #include "fem_stencil.cuh"
+#include "fem_strip.cuh"
 
 #define FEM_MAX_LEVELS 14
 
@@ -23,6 +25,7 @@
 #define SL_PAP 3     // p.Ap
 #define SL_RZ 4      // r.z (direct)
 #define SL_BSUM 5    // sum b (mean-zero rhs)
+#define SL_ZA 6      // r.z of the approximate inverse
 #define SL_BI 6      // BiCGSTAB: 6 rhat.r, 7 rhat.q, 8 s.s, 9 t.s, 10 t.t
 #define SL_LVL0 12
 #define SL_R(n) (SL_LVL0 + 6 * (n))      // 2 slots: sum R_n, sum R_n / D_n
@@ -41,15 +44,19 @@ struct MgLevel {
   FemLattice lat;
   const double* tab;      // assembled stencil of L_e (core/element_calc.py:27)
   const double* tab_off;  // assembled stencil of L_e with zero diagonal (core/multigrid.py:66)
+  int tab_s;              // offset (doubles) of tab in the kernel's shared memory; tab_off, then 1 / diag and
+                          // diag by node class, right behind it
   const double* diag;     // assembled diag(L) (core/element_calc.py:99)
   const double* invD;     // 1 / diag
   const double* winvD;    // 1 / diag, 0 on gamma_p (pinned mode)
   const uint8_t* pin;     // gamma_p mask of this level (pinned mode), else null
+  const uint8_t* mpin;    // the mask that winvD was made from (whole words)
   double sum_invD;        // sum 1 / diag
   double sum_colw;        // sum over nodes of the prolongation column sums (levels >= 1)
   double sum_rc;          // sum over nodes of the restriction row sums c = R 1 (levels >= 1)
   double sum_rcD;         // sum of c / diag
   double inv_nn;          // 1 / nn (means)
+  FemStripPlan pd, pl;    // strips of the down-sweep to the next level and of a whole-lattice phase
   double* x;              // level correction X_n
   double* r;              // level residual R_n (level 0: the CG residual)
   double* t;              // scratch (fine residual before restriction / prolongated x)
@@ -58,15 +65,12 @@ struct MgLevel {
 struct CgArgs {
   FemSync sync;
   int nlev;            // multigrid levels (level 0 = the problem mesh)
-  int block_from;      // first level handled by the coarse-level team (<= nlev - 1)
-  int team;            // CTAs in the coarse-level team (the first ones of the grid)
   int prec;
   int pinned;          // 1: set_zeroP (rows / values on gamma_p zeroed); 0: mean-zero
   int center_rhs;      // mean-zero: subtract mean(b) first (solvers/standard.py:106)
   int maxiter, coarse_maxiter;
   double tol, atol, coarse_tol;
   const double* b;     // rhs (nn)
-  double* bwork;       // centred rhs copy (nn) when center_rhs
   double* x;           // in: x0, out: solution (nn)
   double *r, *z, *p0, *p1, *Ap;
   const uint8_t* ai_pin;  // approx_inv pin set (gamma_p incl. the scalar-0 default)
@@ -74,13 +78,25 @@ struct CgArgs {
   int* status;         // device out: FEM_ERR_* of this solve
   double* final_rr;    // device out: final r.r (diagnostics)
   int post;            // final pin / mean fix of solvers/standard.py:119-123
-  int block_smem_from; // first level of the V-cycle run inside CTA 0 from shared memory (nlev: none)
+  int dense_lv;        // level from which the V-cycle is one dense product (nlev: none)
+  int dense_ld;        // row pitch of dense_C (even, zero-padded)
+  const double* dense_C;  // the V-cycle's operator on that level (row-major)
   MgLevel lv[FEM_MAX_LEVELS];
-  const double* bd[FEM_MAX_LEVELS];  // per-CTA shared-memory copies of those levels' 1/D (0 on gamma_p if pinned)
 };
 
+// Whether a CG solve keeps its partial sums per work item (GridReducer::item_sums):
+// the wall-bounded quad4 solves of the servers, whose bits must not depend on how
+// many CTAs beyond their share a context may use. Elsewhere one column per CTA: a
+// mean-zero solve reads sums in every phase, and 1,184 columns in place of 148 cost
+// each read ~1 us.
+template <int KIND, bool PIN>
+__host__ __device__ constexpr bool fem_items() {
+  return KIND == FEM_Q1_2D && PIN;
+}
+
 __device__ __forceinline__ void fem_zero_partials(const FemSync& s) {
-  for (int k = threadIdx.x; k < FEM_NSLOTS; k += blockDim.x) s.partials[(size_t)k * gridDim.x + blockIdx.x] = 0.0;
+  const int n = FEM_NSLOTS * s.ncols;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) s.partials[k] = 0.0;
 }
 
 // Copy the (param-space) solver arguments into shared memory so that the
@@ -94,60 +110,53 @@ __device__ __forceinline__ void fem_stage_args(const T& src, T* dst) {
   __syncthreads();
 }
 
-// Stencil tables of the solver levels in shared memory (FEM_TAB_SMEM doubles
-// after the tile buffer): copied once per launch, in level order while they
-// fit, and the shared argument copy is pointed at them. Tables that do not fit
-// stay in global memory; every reader uses plain loads, so both work.
-#define FEM_TAB_SMEM 2048
-template <int KIND>
-__device__ void fem_tables_to_smem(CgArgs& sA, double* stab) {
-  constexpr int NOFF = KI<KIND>::NOFF;
-  int off = 0;
+// Tables of the 2D solver levels in shared memory, from `base` doubles into it:
+// the stencils and, per node class, 1 / diag and diag (a uniform mesh has one
+// value per class, so the sweeps read no diagonal from memory). Copied once per
+// launch; the shared argument copy is pointed at them. fem_tab_smem: the doubles
+// they take (host and device).
+__host__ __device__ __forceinline__ int fem_tab_doubles(const FemGrid& g) {
+  return fem_stencil_ncls(g) * fem_stencil_noff(g.kind);
+}
+__host__ __device__ __forceinline__ int fem_level_tab_doubles(const FemGrid& g) {
+  return 2 * fem_tab_doubles(g) + 2 * fem_stencil_ncls(g);
+}
+__host__ __device__ __forceinline__ int fem_tab_smem(const CgArgs& A) {
+  int n = 0;
+  for (int l = 0; l < A.nlev; ++l) n += fem_level_tab_doubles(A.lv[l].g);
+  return n;
+}
+__device__ __forceinline__ void fem_tables_to_smem(CgArgs& sA, double* smem, int base) {
+  int off = base;
   for (int l = 0; l < sA.nlev; ++l) {
     const MgLevel& L = sA.lv[l];
-    if (!L.tab || !L.tab_off) break;
-    const int m = fem_stencil_ncls(L.g) * NOFF;
-    if (off + 2 * m > FEM_TAB_SMEM) break;
+    const FemGrid& g = L.g;
+    const int m = fem_tab_doubles(g);
     for (int q = threadIdx.x; q < m; q += blockDim.x) {
-      stab[off + q] = L.tab[q];
-      stab[off + m + q] = L.tab_off[q];
+      smem[off + q] = L.tab[q];
+      smem[off + m + q] = L.tab_off[q];
     }
-    off += 2 * m;
+    if (g.kind != FEM_HEX8) {
+      const int ncls = fem_stencil_ncls(g), nc = fem_axis_ncls(g.kind, g.periodic);
+      for (int q = threadIdx.x; q < ncls; q += blockDim.x) {
+        const int i = fem_axis_rep(g.kind, g.periodic, q % nc, g.nex), j = fem_axis_rep(g.kind, g.periodic, q / nc, g.ney);
+        const bool has = i >= 0 && j >= 0;
+        smem[off + 2 * m + q] = has ? L.invD[j * g.nnx + i] : 0.0;
+        smem[off + 2 * m + ncls + q] = has ? L.diag[j * g.nnx + i] : 0.0;
+      }
+    }
+    off += fem_level_tab_doubles(g);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    off = 0;
+    off = base;
     for (int l = 0; l < sA.nlev; ++l) {
       MgLevel& L = sA.lv[l];
-      if (!L.tab || !L.tab_off) break;
-      const int m = fem_stencil_ncls(L.g) * NOFF;
-      if (off + 2 * m > FEM_TAB_SMEM) break;
-      L.tab = stab + off;
-      L.tab_off = stab + off + m;
-      off += 2 * m;
-    }
-  }
-  __syncthreads();
-}
-
-// 1/D of the levels that the V-cycle runs inside CTA 0 (pinned: winvD, whose
-// zeros mark gamma_p), copied into this CTA's shared memory once per launch
-// (FEM_BLK_SMEM doubles); sA.bd[l] points at level l's copy.
-#define FEM_BLK_SMEM 2048
-__device__ __forceinline__ void fem_block_levels_to_smem(CgArgs& sA, double* sbd) {
-  int off = 0;
-  for (int l = sA.block_smem_from; l < sA.nlev; ++l) {
-    const MgLevel& L = sA.lv[l];
-    const double* src = sA.pinned ? L.winvD : L.invD;
-    for (int q = threadIdx.x; q < L.g.nn; q += blockDim.x) sbd[off + q] = src[q];
-    off += L.g.nn;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    off = 0;
-    for (int l = sA.block_smem_from; l < sA.nlev; ++l) {
-      sA.bd[l] = sbd + off;
-      off += sA.lv[l].g.nn;
+      const int m = fem_tab_doubles(L.g);
+      L.tab_s = off;
+      L.tab = smem + off;
+      L.tab_off = smem + off + m;
+      off += fem_level_tab_doubles(L.g);
     }
   }
   __syncthreads();
@@ -217,193 +226,141 @@ __device__ __forceinline__ LevelAffine fem_level_affine(const Red& red, const Cg
 
 // Down-sweep step n -> n+1 in one phase: pre-smooth from zero
 // (xh = (2/3) rh / D, 0 on gamma_p or minus its mean), fine residual
-// t = rh - L xh, restriction u_{n+1} = R t. Tiled over the coarse unique lattice
-// (16 coarse columns x CTY rows, CTY chosen for one round of tiles): u and 1/D
-// of the tile's fine region plus the stencil halo, and 1/D of its coarse nodes,
-// are staged in one batch; xh, t (on the region plus one node) and the
-// restriction are then formed from smem only. Each CTA writes x_n and sums t
-// only on the fine nodes its tile owns.
-template <int KIND, bool PIN, class Team, class Red>
-__device__ __noinline__ bool mg_down(const Team& tm, const Red& red, const CgArgs& A, int n, double* smem) {
-  constexpr int R = KI<KIND>::R, W = KI<KIND>::W, NOFF = KI<KIND>::NOFF;
+// t = rh - L xh, restriction u_{n+1} = R t. By warp strips of coarse columns: xh
+// and t live in registers, t's neighbours come by shuffle, and a coarse row is
+// complete with its upper t row; the lane of a coarse node's fine column forms it.
+// Each strip writes x_n and sums t on its coarse columns' own fine columns (2C and
+// 2C + 1). Bound by one pass over u and x_n and by the phase's barrier.
+template <int KIND, bool PIN, bool PER, class Team, class Red>
+__device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const CgArgs& A, int n, double* smem) {
+  constexpr int NC = KS<KIND>::NC, H = KS<KIND>::H, CT = KS<KIND>::COARSE;
   fem_trace_mark(A.sync, 15);
   const MgLevel& L = A.lv[n];
   const MgLevel& C = A.lv[n + 1];
   const FemGrid& g = L.g;
-  const int nn = g.nn;
   constexpr bool pinned = PIN;  // A.pinned, fixed per kernel instantiation
   LevelAffine f{0.0, 0.0, 0.0};
   double mx = 0.0;
-  bool have_f = pinned;
   // the level's affine terms (mean-zero): partial loads issued now, combined
-  // after the first tile's copies have been issued
+  // after the first rows' loads have been issued
   int asl[3];
   fem_level_affine_slots(n, asl);
   typename Red::template Pending<3> pend{};
   if (!pinned) pend = red.template result_begin<3>(asl);
-  fem_trace_mark(A.sync, 16);
-  auto read_affine = [&]() {
-    if (have_f) return;
-    double u3[3];
-    fem_trace_mark(A.sync, 17);
-    red.template result_end<3>(pend, u3, smem);
-    fem_trace_mark(A.sync, 18);
-    f = fem_level_affine_from(A, n, u3);
-    mx = (2.0 / 3.0) * f.sum_rhD * L.inv_nn;
-    if (threadIdx.x == 0) {
-      fem_affine_cache()[2 * n] = f.alpha;
-      fem_affine_cache()[2 * n + 1] = f.beta;
-    }
-    have_f = true;
-  };
-  const double* u = L.r;
-  const double* iDv = pinned ? L.winvD : L.invD;
-  const double* tab = L.tab;
+  const double* __restrict__ u = L.r;
+  const uint8_t* __restrict__ mk = L.mpin;
+  double* __restrict__ xo = L.x;
+  double* __restrict__ cr = C.r;
+  constexpr int per = PER, nc = fem_axis_ncls(KIND, PER);
   const int ux = g.nnx, uy = g.nny;
-  const int nc = fem_axis_ncls(KIND, g.periodic);
   const int cux = C.lat.ux(), cuy = C.lat.uy();
-  const int CTX = 16, ntx = (cux + CTX - 1) / CTX;
-  const int FW = 2 * CTX + 1, SW = FW + 2 * R;
-  // smem per tile: u and xh on SW x SH, t on FW x FH, coarse 1/D on CTX x CTY,
-  // gamma_p flags (bytes) on SW x SH
-  auto need = [&](int cty) {
-    const int fh = 2 * cty + 1, sh = fh + 2 * R;
-    return 2 * SW * sh + FW * fh + CTX * cty + (SW * sh + 7) / 8 + 1;
-  };
-  int CTY;
-  {
-    int nty_t = tm.ncta() / ntx;
-    if (nty_t < 1) nty_t = 1;
-    CTY = (cuy + nty_t - 1) / nty_t;
-    if (CTY > cuy) CTY = cuy;
-    while (CTY > 1 && need(CTY) > FEM_TILE_SMEM) --CTY;
-  }
-  const int FH = 2 * CTY + 1, SH = FH + 2 * R, NS = SW * SH;
-  double* su = smem + 128;
-  double* sx = su + NS;
-  double* st = sx + NS;
-  double* sci = st + FW * FH;
-  unsigned char* spin = reinterpret_cast<unsigned char*>(sci + CTX * CTY);
-  const int nty = (cuy + CTY - 1) / CTY, ntile = ntx * nty;
+  const double* tab = smem + L.tab_s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwt = tm.ncta() * (blockDim.x >> 5);
+  const FemStripPlan P = L.pd;
+  const unsigned ring = fem_ring_lane(smem + 128);
   double acc[3] = {0.0, 0.0, 0.0};  // sum t (owned fine nodes), sum u_{n+1}, sum u_{n+1} / D_{n+1}
-  for (int tl = tm.cta(); tl < ntile; tl += tm.ncta()) {
-    const int by = tl / ntx, bx = tl - by * ntx;
-    const int C0 = bx * CTX, R0 = by * CTY;
-    const int fx0 = 2 * C0 - 1, fy0 = 2 * R0 - 1;  // fine coordinates of the t-region origin
-    auto fidx = [&](int q) -> int {
-      const int ly = q / SW, lx = q - ly * SW;
-      int gx = fx0 - R + lx, gy = fy0 - R + ly;
-      if (g.periodic) {
-        gx = fem_wrap(gx, ux);
-        gy = fem_wrap(gy, uy);
-      } else {
-        gx = gx < 0 ? 0 : (gx >= ux ? ux - 1 : gx);
-        gy = gy < 0 ? 0 : (gy >= uy ? uy - 1 : gy);
-      }
-      return gy * ux + gx;
-    };
-    auto rowb = [&](int r) -> int {
-      int gy = fy0 - R + r;
-      gy = g.periodic ? fem_wrap(gy, uy) : (gy < 0 ? 0 : (gy >= uy ? uy - 1 : gy));
-      return gy * ux;
-    };
-    auto colx = [&](int c) -> int {
-      const int gx = fx0 - R + c;
-      return g.periodic ? fem_wrap(gx, ux) : (gx < 0 ? 0 : (gx >= ux ? ux - 1 : gx));
-    };
-    fem_stage_2d(su, u, SW, SH, rowb, colx);
-    fem_stage_2d(sx, iDv, SW, SH, rowb, colx);
-    fem_stage(sci, C.invD, CTX * CTY, [&](int q) -> int {
-      const int ky = q / CTX, kx = q - ky * CTX;
-      const int Rr = min(R0 + ky, cuy - 1), Cc = min(C0 + kx, cux - 1);
-      return Rr * cux + Cc;
-    });
-    read_affine();
-    fem_trace_mark(A.sync, 1);
-    fem_stage_wait();
-    fem_trace_mark(A.sync, 2);
-    // xh on the staged region (pinned: winvD is 0 on gamma_p, which also marks it)
-    for (int q = threadIdx.x; q < NS; q += blockDim.x) {
-      const double d = sx[q];
-      double v;
-      if (pinned) {
-        spin[q] = (d == 0.0);
-        v = (2.0 / 3.0) * su[q] * d;
-      } else {
-        double rh = su[q] - f.beta;
-        if (n > 0) {
-          const int j = fidx(q), r = j / ux, c = j - r * ux;
-          rh = su[q] - f.alpha * fem_restrict_rowsum(L.lat, r, c) - f.beta;
-        }
-        v = (2.0 / 3.0) * rh * d - mx;
-      }
-      sx[q] = v;
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < FW * FH; q += blockDim.x) {
-      const int py = q / FW, px = q - py * FW;
-      const int x = fx0 + px, y = fy0 + py;
-      double tv = 0.0;
-      if (x >= 0 && x < ux && y >= 0 && y < uy) {
-        const int cx = fem_axis_cls(KIND, g.periodic, x, g.nex), cy = fem_axis_cls(KIND, g.periodic, y, g.ney);
-        const double* cf = tab + (size_t)(cy * nc + cx) * NOFF;
-        double Lx = 0.0;
+  const int sl[3] = {SL_T(n), SL_R(n + 1), SL_R(n + 1) + 1};
+  bool first = true;
+#pragma unroll 1
+  for (int it = warp * tm.ncta() + tm.cta(); first || it < P.nitem; it += nwt) {
+    const bool act = it < P.nitem;
+    int sx, sy;
+    fem_strip_item(P, act ? it : 0, sx, sy);
+    const int R0 = sy * P.seg, R1 = act ? min(cuy, R0 + P.seg) : R0;
+    // a pair starts on its coarse node's fine column; single columns run from one
+    // left of the first coarse node's, after the stencil's halo
+    const FemCols<NC> p(NC == 2 ? 2 * (sx * CT - 1 + lane) : 2 * sx * CT - 1 - H + lane, ux, per);
+    const int Cc = p.x >> 1;  // the coarse column at (an even) p.x
+    const bool own = NC == 2 ? lane >= 1 && lane <= CT : lane > H && lane <= H + 2 * CT;
+    const bool cen = own && (NC == 2 || !(p.x & 1)) && Cc < cux;
+    const double* idt = tab + 2 * fem_tab_doubles(g);  // 1 / D by class
+    int kx[NC];     // the columns' classes
+    double wc[NC];  // and their factors of the row sums
 #pragma unroll
-        for (int dy = 0; dy < W; ++dy)
+    for (int c = 0; c < NC; ++c) {
+      kx[c] = fem_axis_cls(KIND, per, p.g[c], g.nex);
+      wc[c] = fem_restrict_rowsum(L.lat, 0, p.g[c]) / 1.5;
+    }
+    // t rows 2 R0 - 1 .. 2 R1 - 1; those outside the lattice count as zero (the
+    // full-lattice restriction does not reach below row or column 0, periodic or not)
+    const int y0 = 2 * R0 - 1, y1 = act ? 2 * R1 : y0;
+    double dl = 0.0, dc = 0.0, dr = 0.0, ml = 0.0, mc = 0.0, mr = 0.0;  // t of the rows below and at the coarse row
+    fem_strip<KIND, PER, pinned ? 2 * NC : NC, 2, 1>(
+        g, tab, ring, p, y0, y1,
+        [&](int, int row, unsigned slot) {
 #pragma unroll
-          for (int dx = 0; dx < W; ++dx) Lx += cf[dy * W + dx] * sx[(py + dy) * SW + px + dx];
-        const int qc = (py + R) * SW + px + R;
-        double rz;
-        if (pinned) {
-          const bool p = spin[qc] != 0;
-          rz = p ? 0.0 : su[qc];
-          if (p) Lx = 0.0;
-        } else {
-          rz = (n == 0) ? su[qc] - f.beta : su[qc] - f.alpha * fem_restrict_rowsum(L.lat, y, x) - f.beta;
-        }
-        tv = rz - Lx;
-        // fine nodes owned by this tile: [2 C0, 2 C0 + 2 CTX) x [2 R0, 2 R0 + 2 CTY)
-        if (px >= 1 && px <= 2 * CTX && py >= 1 && py <= 2 * CTY) {
-          L.x[y * ux + x] = sx[qc];
-          acc[0] += tv;
-        }
-      }
-      st[q] = tv;
-    }
-    __syncthreads();
-    fem_trace_mark(A.sync, 3);
-    for (int kk = threadIdx.x; kk < CTX * CTY; kk += blockDim.x) {
-      const int ky = kk / CTX, kx = kk - ky * CTX;
-      const int Rr = R0 + ky, Cc = C0 + kx;
-      if (Rr < cuy && Cc < cux) {
-        // fine (2Rr + dr, 2Cc + dc) sits at t-region (1 + 2 ky + dr, 1 + 2 kx + dc)
-        const int cy0 = 1 + 2 * ky, cx0 = 1 + 2 * kx;
-        const int fyc = 2 * Rr, fxc = 2 * Cc;
-        const bool up = fyc + 1 < L.lat.ny, dn = fyc - 1 >= 0, rt = fxc + 1 < L.lat.nx, lf = fxc - 1 >= 0;
-        double e = 0.0, d = 0.0;
-        if (up) e += st[(cy0 + 1) * FW + cx0];
-        if (dn) e += st[(cy0 - 1) * FW + cx0];
-        if (rt) e += st[cy0 * FW + cx0 + 1];
-        if (lf) e += st[cy0 * FW + cx0 - 1];
-        if (up && rt) d += st[(cy0 + 1) * FW + cx0 + 1];
-        if (up && lf) d += st[(cy0 + 1) * FW + cx0 - 1];
-        if (dn && rt) d += st[(cy0 - 1) * FW + cx0 + 1];
-        if (dn && lf) d += st[(cy0 - 1) * FW + cx0 - 1];
-        const double v = st[cy0 * FW + cx0] + 0.5 * e + 0.25 * d;
-        C.r[Rr * cux + Cc] = v;
-        acc[1] += v;
-        acc[2] += v * sci[kk];
-      }
-    }
-    __syncthreads();
+          for (int c = 0; c < NC; ++c) {
+            fem_ring_copy(slot + c * 256, u + row + p.g[c]);
+            if (pinned) fem_ring_copy_mask(slot + (NC + c) * 256, mk, row + p.g[c]);
+          }
+        },
+        [](int, unsigned) {},
+        [&](int c, int, int ry, int i, unsigned slot, double(&car)[2], bool& flag) {
+          const double d = idt[fem_axis_cls(KIND, per, ry, g.ney) * nc + kx[c]];
+          double rh = fem_ring_get(slot), v;
+          if (pinned) {
+            flag = fem_ring_byte(slot + NC * 256, i);
+            v = flag ? 0.0 : (2.0 / 3.0) * rh * d;
+          } else {
+            flag = false;
+            const double wr = (ry == 0 || (!per && ry == uy - 1)) ? 1.5 : 2.0;
+            rh = n > 0 ? rh - f.alpha * (wr * wc[c]) - f.beta : rh - f.beta;
+            v = (2.0 / 3.0) * rh * d - mx;
+          }
+          car[0] = rh;
+          car[1] = v;
+          return v;
+        },
+        [&](int y, const double(&Lx)[NC], const double(&car)[NC][2], const bool(&flag)[NC]) {
+          double tv[NC];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const bool in = p.in[c] && y >= 0 && y < uy;
+            tv[c] = (!in || flag[c]) ? 0.0 : car[c][0] - Lx[c];
+            if (own && in && y >= 2 * R0) {
+              xo[y * ux + p.x + c] = car[c][1];
+              if (!pinned) acc[0] += tv[c];
+            }
+          }
+          const double tl = __shfl_up_sync(0xffffffffu, tv[NC - 1], 1);
+          const double tr = NC == 2 ? tv[NC - 1] : __shfl_down_sync(0xffffffffu, tv[0], 1);
+          if (y & 1) {
+            if (y > 2 * R0 && cen) {  // the t row above coarse row y / 2
+              const double e = ((tv[0] + dc) + mr) + ml, d = ((tr + tl) + dr) + dl;
+              const double v = mc + 0.5 * e + 0.25 * d;
+              const int I = (y >> 1) * cux + Cc;
+              cr[I] = v;
+              if (!pinned) {
+                acc[1] += v;
+                acc[2] += v * C.invD[I];
+              }
+            }
+            dl = tl;
+            dc = tv[0];
+            dr = tr;
+          } else {
+            ml = tl;
+            mc = tv[0];
+            mr = tr;
+          }
+        },
+        [&]() {
+          if (!pinned && first) {
+            double u3[3];
+            red.template result_end<3>(pend, u3, smem);
+            f = fem_level_affine_from(A, n, u3);
+            mx = (2.0 / 3.0) * f.sum_rhD * L.inv_nn;
+            if (threadIdx.x == 0) {
+              fem_affine_cache()[2 * n] = f.alpha;
+              fem_affine_cache()[2 * n + 1] = f.beta;
+            }
+          }
+        });
+    if (!pinned && act) red.template item_sums<fem_items<KIND, PIN>(), 3>(acc, sl, it);
+    first = false;
   }
-  read_affine();  // CTAs without a tile still cache the level's terms for the up-sweep
   fem_trace_mark(A.sync, 4);
-  if (!pinned) {
-    const int sl[3] = {SL_T(n), SL_R(n + 1), SL_R(n + 1) + 1};
-    return tm.template reduce_sync<3>(acc, sl, smem);
-  }
-  return tm.sync();
+  return pinned ? tm.sync() : red.template finish_items<fem_items<KIND, PIN>(), 3>(tm, acc, sl, smem);
 }
 
 // Coarsest level (solution written to L.t). Pinned: CG to coarse_tol with maxiter coarse_maxiter on
@@ -606,475 +563,267 @@ __device__ __forceinline__ void mg_xsums(const MgLevel& L, int i, double xi, dou
 }
 
 // Up-sweep at level n: prolongate X_{n+1}, add to X_n, one weighted Jacobi sweep,
-// in one phase per 32 x TY tile. Staged in one batch: X_n on the tile plus the
-// stencil halo (and ω/D there in pinned mode, whose zeros mark gamma_p), the
-// coarse X_{n+1} under that region, and rhs and diag of the tile's own nodes.
-// The prolongated iterate y = X_n + P X_{n+1} (- means, or 0 on gamma_p) is
-// formed in smem; the sweep then reads smem only. For n == 0 the result is
-// z = M r and the phase also accumulates the r.z pieces.
-template <int KIND, bool PIN, class Team, class Red>
-__device__ __noinline__ bool mg_up(const Team& tm, const Red& red, const CgArgs& A, int n, double* smem) {
-  constexpr int R = KI<KIND>::R, W = KI<KIND>::W, NOFF = KI<KIND>::NOFF;
+// in one phase by warp strips. Per fine row a lane loads X_n, the rhs and, pinned,
+// the gamma_p bytes of its columns, and with every second row the coarse value at
+// or left of its column (the one right of it too, or, of a pair, the next lane's). y = X_n + P X_{n+1}
+// (- means, or 0 on gamma_p) is the stencil's input. For n == 0 the result is
+// z = M r and the phase also accumulates the r.z pieces. Bound by one pass over
+// X_n, rhs and the result, and by the phase's barrier.
+template <int KIND, bool PIN, bool PER, class Team, class Red>
+__device__ __forceinline__ bool mg_up(const Team& tm, const Red& red, const CgArgs& A, int n, double* smem) {
+  constexpr int R = KI<KIND>::R, NC = KS<KIND>::NC, H = KS<KIND>::H;
   fem_trace_mark(A.sync, 14);
   const MgLevel& L = A.lv[n];
   const MgLevel& C = A.lv[n + 1];
   const FemGrid& g = L.g;
-  const int nn = g.nn;
   constexpr bool pinned = PIN;  // A.pinned, fixed per kernel instantiation
   double mX = 0.0, mP = 0.0;
   LevelAffine f{0.0, 0.0, 0.0};
-  bool have_m = pinned;
   // the coarse correction's means (mean-zero): partial loads issued now,
-  // combined after the first tile's copies have been issued
+  // combined after the first rows' loads have been issued
   const int msl[2] = {SL_X(n + 1), SL_X(n + 1) + 1};
   typename Red::template Pending<2> pend{};
   if (!pinned) pend = red.template result_begin<2>(msl);
-  auto read_means = [&]() {
-    if (have_m) return;
-    double v[2];
-    red.template result_end<2>(pend, v, smem);  // its __syncthreads also publishes the cache
-    mX = v[0] * C.inv_nn;
-    mP = (v[1] - mX * C.sum_colw) * L.inv_nn;
-    if (n > 0) {
-      f.alpha = fem_affine_cache()[2 * n];
-      f.beta = fem_affine_cache()[2 * n + 1];
-    }
-    have_m = true;
-  };
+  const double* __restrict__ xi = L.x;
+  const double* __restrict__ rr = L.r;
+  const double* __restrict__ xc = C.t;
+  const uint8_t* __restrict__ mk = L.mpin;
+  double* __restrict__ to = L.t;
+  constexpr int per = PER, nc = fem_axis_ncls(KIND, PER);
   const int ux = g.nnx, uy = g.nny, cux = C.lat.ux(), cuy = C.lat.uy();
-  const bool per = g.periodic;
-  const int nc = fem_axis_ncls(KIND, per);
-  const int WR = blockDim.x >> 5, tx = threadIdx.x & 31, ty0 = threadIdx.x >> 5;
-  const int SX = 32 + 2 * R, CXB = SX / 2 + 3;
-  const int nf = pinned ? 2 : 1;
-  auto need = [&](int ty) { return nf * SX * (ty + 2 * R) + CXB * ((ty + 2 * R) / 2 + 3) + 64 * ty; };
-  const int ntx = (ux + 31) >> 5;
-  int TY;
-  {
-    int nty_t = tm.ncta() / ntx;
-    if (nty_t < 1) nty_t = 1;
-    TY = (uy + nty_t - 1) / nty_t;
-    const int minr = WR < uy ? WR : uy;
-    if (TY < minr) TY = minr;
-    if (TY > uy) TY = uy;
-    while (TY > 1 && need(TY) > FEM_TILE_SMEM) --TY;
-  }
-  const int SY = TY + 2 * R, NS = SX * SY, CYB = SY / 2 + 3;
-  double* sy = smem + 128;
-  double* sw = sy + NS;                     // pinned only
-  double* sc = sy + nf * NS;                // coarse X_{n+1}, CXB x CYB
-  double* sr = sc + CXB * CYB;              // rhs of owned nodes, 32 x TY
-  double* sd = sr + 32 * TY;                // 1 / diag of owned nodes
-  const int nty = (uy + TY - 1) / TY, ntile = ntx * nty;
-  const double* tabo = L.tab_off;
+  const double* tab = smem + L.tab_s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwt = tm.ncta() * (blockDim.x >> 5);
+  const FemStripPlan P = L.pl;
+  const unsigned ring = fem_ring_lane(smem + 128);
   const double w = 2.0 / 3.0;
-  double a[2] = {0.0, 0.0};
-  for (int tl = tm.cta(); tl < ntile; tl += tm.ncta()) {
-    const int by = tl / ntx, bx = tl - by * ntx;
-    const int x0 = bx * 32, y0 = by * TY, gx0 = x0 - R, gy0 = y0 - R;
-    const int cr0 = fem_floordiv2(gy0), cc0 = fem_floordiv2(gx0);
-    // fine coordinates of a staged point: unwrapped (periodic) or clamped
-    auto fcoord = [&](int q, int& fr, int& fc) {
-      const int ly = q / SX, lx = q - ly * SX;
-      fr = gy0 + ly;
-      fc = gx0 + lx;
-      if (!per) {
-        fr = fr < 0 ? 0 : (fr >= uy ? uy - 1 : fr);
-        fc = fc < 0 ? 0 : (fc >= ux ? ux - 1 : fc);
-      }
-    };
-    auto fidx = [&](int q) -> int {
-      int fr, fc;
-      fcoord(q, fr, fc);
-      if (per) {
-        fr = fem_wrap(fr, uy);
-        fc = fem_wrap(fc, ux);
-      }
-      return fr * ux + fc;
-    };
-    auto oidx = [&](int q) -> int {  // owned node q = ty * 32 + tx, clamped into the lattice
-      const int ty = q >> 5, x = min(x0 + (q & 31), ux - 1), y = min(y0 + ty, uy - 1);
-      return y * ux + x;
-    };
-    auto rowb = [&](int r) -> int {
-      int fr = gy0 + r;
-      fr = per ? fem_wrap(fr, uy) : (fr < 0 ? 0 : (fr >= uy ? uy - 1 : fr));
-      return fr * ux;
-    };
-    auto colx = [&](int c) -> int {
-      const int fc = gx0 + c;
-      return per ? fem_wrap(fc, ux) : (fc < 0 ? 0 : (fc >= ux ? ux - 1 : fc));
-    };
-    fem_stage_2d(sy, L.x, SX, SY, rowb, colx);
-    if (pinned) fem_stage_2d(sw, L.winvD, SX, SY, rowb, colx);
-    fem_stage(sc, C.t, CXB * CYB, [&](int q) -> int {
-      const int i = q / CXB, j = q - i * CXB;
-      int cr = cr0 + i, cc = cc0 + j;
-      if (per) {
-        cr = fem_wrap(cr, cuy);
-        cc = fem_wrap(cc, cux);
-      } else {
-        cr = cr < 0 ? 0 : (cr >= cuy ? cuy - 1 : cr);
-        cc = cc < 0 ? 0 : (cc >= cux ? cux - 1 : cc);
-      }
-      return cr * cux + cc;
-    });
-    fem_stage(sr, L.r, 32 * TY, oidx);
-    fem_stage(sd, L.invD, 32 * TY, oidx);
-    read_means();
-    fem_trace_mark(A.sync, 11);
-    fem_stage_wait();
-    // y = X_n + P X_{n+1} in place (the arithmetic of fem_interp_at)
-    for (int q = threadIdx.x; q < NS; q += blockDim.x) {
-      int fr, fc;
-      fcoord(q, fr, fc);
-      double y;
-      if (pinned && sw[q] == 0.0) {
-        y = 0.0;
-      } else {
-        const int Rr = fem_floordiv2(fr) - cr0, Cc = fem_floordiv2(fc) - cc0;
-        auto xH = [&](int dr, int dc) -> double {
-          const double v = sc[(Rr + dr) * CXB + Cc + dc];
-          return pinned ? v : v - mX;
-        };
-        double xh;
-        if (!(fr & 1) && !(fc & 1)) xh = xH(0, 0);
-        else if (!(fr & 1)) xh = 0.5 * xH(0, 0) + 0.5 * xH(0, 1);
-        else if (!(fc & 1)) xh = 0.5 * xH(0, 0) + 0.5 * xH(1, 0);
-        else xh = 0.25 * xH(0, 0) + 0.25 * xH(0, 1) + 0.25 * xH(1, 0) + 0.25 * xH(1, 1);
-        y = sy[q] + (pinned ? xh : xh - mP);
-      }
-      sy[q] = y;
-    }
-    __syncthreads();
-    // Jacobi: x = w (rh - Loff y)/D + (1-w) y on the owned nodes
-    for (int ty = ty0; ty < TY; ty += WR) {
-      const int x = x0 + tx, yy = y0 + ty;
-      if (x < ux && yy < uy) {
-        const int cx = fem_axis_cls(KIND, per, x, g.nex), cy = fem_axis_cls(KIND, per, yy, g.ney);
-        const double* cf = tabo + (size_t)(cy * nc + cx) * NOFF;
-        double off = 0.0;
+  double a[2] = {0.0, 0.0};  // sums of the new iterate
+  const int sl[2] = {SL_X(n), SL_X(n) + 1};
+  bool first = true;
+#pragma unroll 1
+  for (int it = warp * tm.ncta() + tm.cta(); first || it < P.nitem; it += nwt) {
+    const bool act = it < P.nitem;
+    int sx, sy;
+    fem_strip_item(P, act ? it : 0, sx, sy);
+    const FemCols<NC> p(sx * KS<KIND>::OWN + NC * (lane - H), ux, per);
+    const bool own = lane >= H && lane < 32 - H;
+    const int y0 = sy * P.seg, y1 = act ? min(uy, y0 + P.seg) : y0;
+    const double* idt = tab + 2 * fem_tab_doubles(g);  // 1 / D by class
+    int kx[NC];     // the columns' classes
+    double wc[NC];  // and their factors of the row sums
 #pragma unroll
-        for (int dy = 0; dy < W; ++dy)
-#pragma unroll
-          for (int dx = 0; dx < W; ++dx) off += cf[dy * W + dx] * sy[(ty + dy) * SX + tx + dx];
-        const int qc = (ty + R) * SX + tx + R;
-        const double yi = sy[qc];
-        const double rhv = sr[ty * 32 + tx];
-        const double rv = (!pinned && n > 0) ? rhv - f.alpha * fem_restrict_rowsum(L.lat, yy, x) - f.beta : rhv;
-        double xn = w * (rv - off) * sd[ty * 32 + tx] + (1.0 - w) * yi;
-        if (pinned && sw[qc] == 0.0) xn = 0.0;
-        L.t[yy * ux + x] = xn;
-        if (n == 0) {
-          a[0] += xn;
-          a[1] += rhv * xn;
-        } else {
-          a[0] += xn;
-          a[1] += fem_interp_colsum(L.lat, yy, x) * xn;
-        }
-      }
+    for (int c = 0; c < NC; ++c) {
+      kx[c] = fem_axis_cls(KIND, per, p.g[c], g.nex);
+      wc[c] = fem_restrict_rowsum(L.lat, 0, p.g[c]) / 1.5;
     }
-    __syncthreads();
+    const int ca = fem_strip_coord(p.x >> 1, cux, per);        // coarse columns at or left of p.x
+    const int cb = fem_strip_coord((p.x + 1) >> 1, cux, per);  // and at or right of it
+    // X_{n+1} on the coarse columns left and right, on the coarse row at or below
+    // the current fine row (h0) and, on odd rows, above it (h1)
+    double h0a = 0.0, h0b = 0.0, h1a = 0.0, h1b = 0.0;
+    // slots: X_n, rhs, mask, and the coarse row above an odd row (a run that starts
+    // on an odd row takes the one below from memory, one that starts on an even
+    // row its own)
+    constexpr int XC = 2 * NC * 256, MK = XC + (3 - NC) * 256;  // of the coarse values and the mask
+    fem_strip<KIND, PER, 2 * NC + (3 - NC) + (pinned ? NC : 0), 2, 0>(
+        g, tab + fem_tab_doubles(g), ring, p, y0, y1,
+        [&](int y, int row, unsigned slot) {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            fem_ring_copy(slot + c * 256, xi + row + p.g[c]);
+            fem_ring_copy(slot + (NC + c) * 256, rr + row + p.g[c]);
+            if (pinned) fem_ring_copy_mask(slot + MK + c * 256, mk, row + p.g[c]);
+          }
+          if ((y & 1) || y == y0 - R) {
+            const double* src = xc + fem_strip_near((y + 1) >> 1, cuy, per) * cux;
+            fem_ring_copy(slot + XC, src + ca);
+            if (NC == 1) fem_ring_copy(slot + XC + 256, src + cb);
+            if (y == y0 - R && (y & 1)) {
+              src = xc + fem_strip_near(y >> 1, cuy, per) * cux;
+              h0a = src[ca];
+              h0b = src[cb];
+            }
+          }
+        },
+        [&](int y, unsigned slot) {
+          const bool odd = y & 1, start = y == y0 - R;
+          if (NC == 2 && start && odd) h0b = __shfl_down_sync(0xffffffffu, h0a, 1);
+          if (odd || start) {
+            h1a = fem_ring_get(slot + XC);
+            h1b = NC == 2 ? __shfl_down_sync(0xffffffffu, h1a, 1) : fem_ring_get(slot + XC + 256);
+          }
+          if (!odd) {  // the coarse row of the odd row before, or the run's own
+            h0a = h1a;
+            h0b = h1b;
+          }
+        },
+        [&](int c, int y, int, int i, unsigned slot, double(&car)[2], bool& flag) {
+          const double x00 = pinned ? h0a : h0a - mX, x01 = pinned ? h0b : h0b - mX;
+          const bool odd_x = NC == 2 ? c == 1 : p.x & 1;
+          double xh;
+          if (!(y & 1)) {
+            xh = odd_x ? 0.5 * x00 + 0.5 * x01 : x00;
+          } else {
+            const double x10 = pinned ? h1a : h1a - mX, x11 = pinned ? h1b : h1b - mX;
+            xh = odd_x ? 0.25 * x00 + 0.25 * x01 + 0.25 * x10 + 0.25 * x11 : 0.5 * x00 + 0.5 * x10;
+          }
+          flag = pinned && fem_ring_byte(slot + MK, i);
+          const double v = flag ? 0.0 : fem_ring_get(slot) + (pinned ? xh : xh - mP);
+          car[0] = v;
+          car[1] = fem_ring_get(slot + NC * 256);
+          return v;
+        },
+        [&](int y, const double(&off)[NC], const double(&car)[NC][2], const bool(&flag)[NC]) {
+          const double wr = (y == 0 || (!per && y == uy - 1)) ? 1.5 : 2.0;
+          const double* idr = idt + fem_axis_cls(KIND, per, y, g.ney) * nc;
+#pragma unroll
+          for (int c = 0; c < NC; ++c)
+            if (own && p.in[c]) {
+              const double rv = (!pinned && n > 0) ? car[c][1] - f.alpha * (wr * wc[c]) - f.beta : car[c][1];
+              const double xn = flag[c] ? 0.0 : w * (rv - off[c]) * idr[kx[c]] + (1.0 - w) * car[c][0];
+              to[y * ux + p.x + c] = xn;
+              if (n == 0) {
+                a[0] += xn;
+                a[1] += car[c][1] * xn;
+              } else if (!pinned) {
+                a[0] += xn;
+                a[1] += (per ? 4.0 : wr * wc[c]) * xn;
+              }
+            }
+        },
+        [&]() {
+          if (!pinned && first) {
+            double v[2];
+            red.template result_end<2>(pend, v, smem);  // its __syncthreads also publishes the cache
+            mX = v[0] * C.inv_nn;
+            mP = (v[1] - mX * C.sum_colw) * L.inv_nn;
+            if (n > 0) {
+              f.alpha = fem_affine_cache()[2 * n];
+              f.beta = fem_affine_cache()[2 * n + 1];
+            }
+          }
+        });
+    if ((n == 0 || !pinned) && act) red.template item_sums<fem_items<KIND, PIN>(), 2>(a, sl, it);
+    first = false;
   }
   fem_trace_mark(A.sync, 12);
-  if (n == 0 || !pinned) {
-    const int sl[2] = {SL_X(n), SL_X(n) + 1};
-    return tm.template reduce_sync<2>(a, sl, smem);
-  }
-  return tm.sync();
+  return (n > 0 && pinned) ? tm.sync() : red.template finish_items<fem_items<KIND, PIN>(), 2>(tm, a, sl, smem);
 }
 
 // ---------------------------------------------------------------------------
-// The coarse end of the V-cycle inside one CTA, vectors in shared memory
+// The coarse end of the V-cycle as one dense product
 // ---------------------------------------------------------------------------
-// Levels s = A.block_smem_from .. N-1 run in CTA 0 with __syncthreads only,
-// as core/multigrid.py:231-330 writes them (explicit means, no lazy affine
-// terms): no grid or team barrier and no global-memory round trip inside.
-// In: u_s = R t_{s-1} (lv[s].r, raw, from the phase that restricted it) and,
-// mean-zero, the sum of t_{s-1} (slot SL_T(s-1)). Out: the level's corrected
-// X_s in lv[s].t and, mean-zero, its sums in SL_X(s) (CTA 0's column; the
-// other columns of that slot stay zero), which the up-sweep of level s-1
-// consumes as it would a team level's. Vectors r_l, x_l of every block level
-// and one scratch sit in the tile region after the coarse warp CG's p buffer.
-
-// stencil of level L (table tab) at unique node (ix, iy) on the unique-lattice
-// vector v (wrapped, or clamped where the table's coefficient is zero)
-template <int KIND>
-__device__ __forceinline__ double mg_blk_stencil(const MgLevel& L, const double* __restrict__ tab,
-                                                 const double* __restrict__ v, int ix, int iy) {
-  constexpr int R = KI<KIND>::R, W = KI<KIND>::W, NOFF = KI<KIND>::NOFF;
-  const FemGrid& g = L.g;
-  const int per = g.periodic, nnx = g.nnx, nny = g.nny;
-  const int nc = fem_axis_ncls(KIND, per);
-  const double* c = tab + (size_t)(fem_axis_cls(KIND, per, iy, g.ney) * nc + fem_axis_cls(KIND, per, ix, g.nex)) * NOFF;
-  double y = 0.0;
-#pragma unroll
-  for (int dy = 0; dy < W; ++dy) {
-    int w = iy + dy - R;
-    w = per ? fem_wrap(w, nny) : min(max(w, 0), nny - 1);
-#pragma unroll
-    for (int dx = 0; dx < W; ++dx) {
-      int u = ix + dx - R;
-      u = per ? fem_wrap(u, nnx) : min(max(u, 0), nnx - 1);
-      y += c[dy * W + dx] * v[w * nnx + u];
-    }
-  }
-  return y;
-}
-
-// R t at coarse unique node (Rr, Cc) of the level below F (the sums of mg_down)
-__device__ __forceinline__ double mg_blk_restrict(const FemLattice& F, const double* __restrict__ t, int Rr, int Cc) {
-  const int fy = 2 * Rr, fx = 2 * Cc, ux = F.ux(), uy = F.uy();
-  const bool up = fy + 1 < F.ny, dn = fy - 1 >= 0, rt = fx + 1 < F.nx, lf = fx - 1 >= 0;
-  auto at = [&](int y, int x) -> double {
-    y = y >= uy ? y - uy : y;
-    x = x >= ux ? x - ux : x;
-    return t[y * ux + x];
-  };
-  double e = 0.0, d = 0.0;
-  if (up) e += at(fy + 1, fx);
-  if (dn) e += at(fy - 1, fx);
-  if (rt) e += at(fy, fx + 1);
-  if (lf) e += at(fy, fx - 1);
-  if (up && rt) d += at(fy + 1, fx + 1);
-  if (up && lf) d += at(fy + 1, fx - 1);
-  if (dn && rt) d += at(fy - 1, fx + 1);
-  if (dn && lf) d += at(fy - 1, fx - 1);
-  return at(fy, fx) + 0.5 * e + 0.25 * d;
-}
-
-// P x at fine unique node (fr, fc) from the coarse unique-lattice vector x
-// (core/multigrid.py:90-140, the arithmetic of mg_up)
-__device__ __forceinline__ double mg_blk_prolong(const FemLattice& C, const double* __restrict__ x, int fr, int fc) {
-  const int cux = C.ux(), cuy = C.uy(), Rr = fr >> 1, Cc = fc >> 1;
-  auto xH = [&](int dr, int dc) -> double {
-    int r = Rr + dr, c = Cc + dc;
-    r = r >= cuy ? r - cuy : r;
-    c = c >= cux ? c - cux : c;
-    return x[r * cux + c];
-  };
-  if (!(fr & 1) && !(fc & 1)) return xH(0, 0);
-  if (!(fr & 1)) return 0.5 * xH(0, 0) + 0.5 * xH(0, 1);
-  if (!(fc & 1)) return 0.5 * xH(0, 0) + 0.5 * xH(1, 0);
-  return 0.25 * xH(0, 0) + 0.25 * xH(0, 1) + 0.25 * xH(1, 0) + 0.25 * xH(1, 1);
-}
-
-// mean of a block-local sum (every thread gets it)
-__device__ __forceinline__ double mg_blk_mean(double v, int nn, double* smem) {
-  double a[1] = {v};
-  fem_block_sum<1>(a, smem);
-  return a[0] / nn;
-}
-
+// From a level of n nodes down, the V-cycle is a fixed linear map C of the
+// level's residual: the smoothers, transfers and mean removals are linear and
+// the coarsest solve is the inverse (pinned) or one Jacobi sweep (mean-zero). C
+// is formed once per hierarchy (k_dense.cu) and applied here in one phase over
+// the whole grid, where the levels themselves take two phases each plus the
+// coarsest solve. Bound by the load of C from L2 (n^2 doubles over the grid)
+// and one grid barrier.
+//
+// In: u_d = R t_{d-1} (lv[d].r, raw) and, mean-zero, the sum of t_{d-1} (slot
+// SL_T(d-1)); C removes constants itself, so only the alpha c part of the
+// level's affine form is subtracted. Out: X_d in lv[d].t and its sums in
+// SL_X(d), as mg_up leaves them (d == 0: z = M r with the r.z pieces).
+// One warp per row, rows in blocks of 8 (a CTA's warps; a block's sums are one
+// partial column), each lane 16-byte pieces of its row, up to 8 in flight.
 template <int KIND, bool PIN>
-__device__ __noinline__ void mg_block_levels(const GridReducer& gr, const CgArgs& A, double* smem) {
-  const BlockTeam tm;
-  const int N = A.nlev, s = A.block_smem_from;
-  const double w = 2.0 / 3.0;
-  double* base = smem + 128 + FEM_COARSE_WARP_NN;
-  // r_l at base + ro(l), x_l right after it; the scratch after the last level
-  auto ro = [&](int l) {
-    int o = 0;
-    for (int m = s; m < l; ++m) o += 2 * A.lv[m].g.nn;
-    return o;
-  };
-  double* tv = base + ro(N);
-  // 1. the stored rhs of level s: u_s (pinned), or R(t - mean t) - its mean
-  {
-    const MgLevel& L = A.lv[s];
-    const int nn = L.g.nn, ux = L.lat.ux();
-    double* r = base + ro(s);
+__device__ __forceinline__ bool mg_dense(const GridTeam& gt, const GridReducer& gr, const CgArgs& A, double* smem) {
+  const int d = A.dense_lv, ld = A.dense_ld, h = ld >> 1;
+  const MgLevel& L = A.lv[d];
+  const int n = L.g.nn, nblk = (n + 7) >> 3;
+  double a[2] = {0.0, 0.0};
+  const int slx[2] = {SL_X(d), SL_X(d) + 1};
+  if (gt.cta() < nblk) {
+    double* sr = smem + 128;  // u_d (ld doubles), then the results of a block of rows
+    double* sz = sr + ld;
+    fem_stage(sr, L.r, n, [](int q) { return q; });
+    for (int q = n + threadIdx.x; q < ld; q += blockDim.x) sr[q] = 0.0;
     double alpha = 0.0;
-    if (!PIN) {
-      const int sl[1] = {SL_T(s - 1)};
+    if (!PIN && d > 0) {
+      const int sl[1] = {SL_T(d - 1)};
       double u[1];
       gr.result_slots<1>(u, sl, smem);
-      alpha = u[0] * A.lv[s - 1].inv_nn;
+      alpha = u[0] * A.lv[d - 1].inv_nn;
     }
-    double a = 0.0;
-    for (int i = tm.rank(); i < nn; i += tm.size()) {
-      double v = L.r[i];
-      if (!PIN) v -= alpha * fem_restrict_rowsum(L.lat, i / ux, i % ux);
-      r[i] = v;
-      a += v;
+    fem_stage_wait();
+    const int ux = L.lat.ux();
+    if (!PIN && d > 0) {
+      for (int q = threadIdx.x; q < n; q += blockDim.x) sr[q] -= alpha * fem_restrict_rowsum(L.lat, q / ux, q % ux);
+      __syncthreads();
     }
-    if (!PIN) {
-      const double beta = mg_blk_mean(a, nn, smem);
-      for (int i = tm.rank(); i < nn; i += tm.size()) r[i] -= beta;
-    }
-    __syncthreads();
-  }
-  // 2. down: pre-smooth from zero, residual, restriction
-  for (int n = s; n < N - 1; ++n) {
-    const MgLevel& L = A.lv[n];
-    const MgLevel& C = A.lv[n + 1];
-    const int nn = L.g.nn, ux = L.lat.ux(), cux = C.lat.ux(), cnn = C.g.nn;
-    const double* __restrict__ d = A.bd[n];
-    double* r = base + ro(n);
-    double* x = r + nn;
-    double* rc = base + ro(n + 1);
-    const double mr = PIN ? 0.0 : mg_blk_mean([&] {
-      double a = 0.0;
-      for (int i = tm.rank(); i < nn; i += tm.size()) a += r[i];
-      return a;
-    }(), nn, smem);
-    double a = 0.0;
-    for (int i = tm.rank(); i < nn; i += tm.size()) {
-      const double rh = PIN ? (d[i] == 0.0 ? 0.0 : r[i]) : r[i] - mr;
-      const double xh = w * rh * d[i];
-      tv[i] = rh;
-      x[i] = xh;
-      a += xh;
-    }
-    if (!PIN) {
-      const double mx = mg_blk_mean(a, nn, smem);
-      for (int i = tm.rank(); i < nn; i += tm.size()) x[i] -= mx;
-    }
-    __syncthreads();
-    a = 0.0;
-    for (int i = tm.rank(); i < nn; i += tm.size()) {
-      double Lx = mg_blk_stencil<KIND>(L, L.tab, x, i % ux, i / ux);
-      if (PIN && d[i] == 0.0) Lx = 0.0;
-      const double t = tv[i] - Lx;
-      tv[i] = t;
-      a += t;
-    }
-    if (!PIN) {
-      const double mt = mg_blk_mean(a, nn, smem);
-      for (int i = tm.rank(); i < nn; i += tm.size()) tv[i] -= mt;
-    }
-    __syncthreads();
-    a = 0.0;
-    for (int I = tm.rank(); I < cnn; I += tm.size()) {
-      const double v = mg_blk_restrict(L.lat, tv, I / cux, I % cux);
-      rc[I] = v;
-      a += v;
-    }
-    if (!PIN) {
-      const double mh = mg_blk_mean(a, cnn, smem);
-      for (int I = tm.rank(); I < cnn; I += tm.size()) rc[I] -= mh;
-    }
-    __syncthreads();
-  }
-  // 3. coarsest level: one Jacobi sweep from zero (mean-zero) or the warp CG (pinned)
-  {
-    const MgLevel& L = A.lv[N - 1];
-    const int nn = L.g.nn;
-    const double* __restrict__ d = A.bd[N - 1];
-    double* r = base + ro(N - 1);
-    double* x = r + nn;
-    if (!PIN) {
-      double a = 0.0;
-      for (int i = tm.rank(); i < nn; i += tm.size()) a += r[i];
-      const double mr = mg_blk_mean(a, nn, smem);
-      a = 0.0;
-      for (int i = tm.rank(); i < nn; i += tm.size()) {
-        const double v = w * (r[i] - mr) * d[i];
-        x[i] = v;
-        a += v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, bw = blockDim.x >> 8;  // row blocks at a time
+    const double2* __restrict__ v2 = reinterpret_cast<const double2*>(sr);
+#pragma unroll 1
+    for (int b0 = gt.cta(); b0 < nblk; b0 += bw * gt.ncta()) {
+      const int blk = b0 + (warp >> 3) * gt.ncta(), i = blk * 8 + (warp & 7);
+      double s0 = 0.0, s1 = 0.0;
+      if (blk < nblk && i < n) {
+        const double2* __restrict__ row = reinterpret_cast<const double2*>(A.dense_C + (size_t)i * ld);
+        for (int c = lane; c < h; c += 8 * 32) {
+          double2 m[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) m[u] = (c + 32 * u < h) ? __ldg(row + c + 32 * u) : make_double2(0.0, 0.0);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const double2 v = (c + 32 * u < h) ? v2[c + 32 * u] : make_double2(0.0, 0.0);
+            s0 += m[u].x * v.x;
+            s1 += m[u].y * v.y;
+          }
+        }
+        s0 = fem_warp_sum(s0 + s1);
+        if (lane == 0) L.t[i] = s0;
       }
-      const double mx = mg_blk_mean(a, nn, smem);
-      for (int i = tm.rank(); i < nn; i += tm.size()) x[i] -= mx;
-    } else if constexpr (PIN && KIND != FEM_HEX8) {
-      for (int i = tm.rank(); i < nn; i += tm.size()) L.r[i] = r[i];
-      __syncthreads();
-      if (threadIdx.x < 32) mg_coarse_warp<KIND>(A, smem + 128);
-      __syncthreads();
-      for (int i = tm.rank(); i < nn; i += tm.size()) x[i] = L.t[i];
-    }
-    __syncthreads();
-  }
-  // 4. up: prolongate, add, one weighted Jacobi sweep
-  for (int n = N - 2; n >= s; --n) {
-    const MgLevel& L = A.lv[n];
-    const MgLevel& C = A.lv[n + 1];
-    const int nn = L.g.nn, ux = L.lat.ux();
-    const double* __restrict__ d = A.bd[n];
-    double* r = base + ro(n);
-    double* x = r + nn;
-    const double* xc = base + ro(n + 1) + C.g.nn;
-    double a = 0.0;
-    for (int i = tm.rank(); i < nn; i += tm.size()) {
-      const double p = mg_blk_prolong(C.lat, xc, i / ux, i % ux);
-      tv[i] = p;
-      a += p;
-    }
-    const double mp = PIN ? 0.0 : mg_blk_mean(a, nn, smem);
-    for (int i = tm.rank(); i < nn; i += tm.size()) {
-      const double y = x[i] + (tv[i] - mp);
-      tv[i] = (PIN && d[i] == 0.0) ? 0.0 : y;
-    }
-    __syncthreads();
-    a = 0.0;
-    for (int i = tm.rank(); i < nn; i += tm.size()) {
-      const double off = mg_blk_stencil<KIND>(L, L.tab_off, tv, i % ux, i / ux);
-      double xn = w * (r[i] - off) * d[i] + (1.0 - w) * tv[i];
-      if (PIN && d[i] == 0.0) xn = 0.0;
-      x[i] = xn;
-      a += xn;
-    }
-    if (!PIN) {
-      const double mj = mg_blk_mean(a, nn, smem);
-      for (int i = tm.rank(); i < nn; i += tm.size()) x[i] -= mj;
-    }
-    __syncthreads();
-  }
-  // 5. X_s out, with its sums for the level above (mean-zero)
-  {
-    const MgLevel& L = A.lv[s];
-    const int nn = L.g.nn, ux = L.lat.ux();
-    const double* x = base + ro(s) + nn;
-    double a[2] = {0.0, 0.0};
-    for (int i = tm.rank(); i < nn; i += tm.size()) {
-      const double v = x[i];
-      L.t[i] = v;
-      if (!PIN) {
-        a[0] += v;
-        a[1] += fem_interp_colsum(L.lat, i / ux, i % ux) * v;
+      if (d == 0 || !PIN) {
+        if (lane == 0) sz[warp] = s0;
+        __syncthreads();
+        if ((warp & 7) == 0 && blk < nblk) {  // the block's first warp sums its 8 rows
+          const int k = blk * 8 + lane;
+          if (lane < 8 && k < n) {
+            const double z = sz[warp + lane];
+            a[0] += z;
+            a[1] += (d == 0 ? sr[k] : fem_interp_colsum(L.lat, k / ux, k % ux)) * z;
+          }
+          gr.item_sums<fem_items<KIND, PIN>(), 2>(a, slx, blk);
+        }
+        __syncthreads();
       }
     }
-    if (!PIN) gr.reduce<2>(a, SL_X(s), smem);
-    __syncthreads();
   }
+  fem_trace_mark(A.sync, 8);
+  return (d > 0 && PIN) ? gt.sync() : gr.finish_items<fem_items<KIND, PIN>(), 2>(gt, a, slx, smem);
 }
 
 // Full V-cycle on r = lv[0].r; result in lv[0].t (raw; mean-zero subtracts
-// SL_X(0)[0]/nn lazily). Levels < block_from run on the whole grid; levels from
-// block_from down run on the team of the first A.team CTAs (GridTeam::team barriers,
-// data in global memory), the coarsest solve in CTA 0. Grid-produced sums are
-// read over all CTA columns; team phases write only the team's columns (the
-// rest of those slots stay zero), so the same reads stay exact.
-template <int KIND, bool PIN>
-__device__ __noinline__ bool mg_vcycle(const GridTeam& gt, const GridReducer& gr, const CgArgs& A, double* smem,
-                                       unsigned int* team_round, double* cg_r, double* cg_p, double* cg_q) {
-  const int N = A.nlev, s = A.block_from;
+// SL_X(0)[0]/nn lazily). Every level runs on the whole grid, down to the dense
+// coarse operator's level or, without one, to the coarsest, which CTA 0 solves.
+// Grid-produced sums are read over all CTA columns; CTA 0's coarsest sums leave
+// the other columns of their slots zero, so the same reads stay exact.
+//
+// The phases are inlined at one call site each: as functions they saved up to
+// 550 bytes of callee-saved registers per thread and call, 280 KB per CTA, which
+// the barriers' acquires evict from L1.
+template <int KIND, bool PIN, bool PER>
+__device__ __forceinline__ bool mg_vcycle(const GridTeam& gt, const GridReducer& gr, const CgArgs& A, double* smem,
+                                          double* cg_r, double* cg_p, double* cg_q) {
+  static_assert(KIND != FEM_HEX8, "the hex8 multigrid is k_mg3.cu");
+  const int N = A.nlev;
+  const bool dense = A.dense_lv < N;
+  const int s = dense ? A.dense_lv : N - 1;
+#pragma unroll 1
   for (int n = 0; n < s; ++n)
-    if (!mg_down<KIND, PIN>(gt, gr, A, n, smem)) return false;
-  const int b = A.block_smem_from < N ? A.block_smem_from : N - 1;  // team levels: [s, b)
-  if ((int)blockIdx.x < A.team) {
-    const GridTeam tt = GridTeam::team(gt.s, team_round, A.team);
-    for (int n = s; n < b; ++n)
-      if (!mg_down<KIND, PIN>(tt, gr, A, n, smem)) return false;
-    fem_trace_mark(A.sync, 7);
-    if (b < N - 1 || A.block_smem_from == N - 1) {
-      // levels b.. inside CTA 0 from shared memory (2D)
-      if constexpr (KIND != FEM_HEX8) {
-        if (blockIdx.x == 0) mg_block_levels<KIND, PIN>(gr, A, smem);
-      }
-      fem_trace_mark(A.sync, 8);
-    } else if (blockIdx.x == 0) {
-      bool warp_solve = false;
-      if constexpr (PIN && KIND != FEM_HEX8) warp_solve = A.lv[N - 1].g.nn <= FEM_COARSE_WARP_NN;
-      if (warp_solve) {
-        if constexpr (PIN && KIND != FEM_HEX8) {
-          if (threadIdx.x < 32) mg_coarse_warp<KIND>(A, smem + 128);
-        }
+    if (!mg_down<KIND, PIN, PER>(gt, gr, A, n, smem)) return false;
+  if (dense) {
+    if (!mg_dense<KIND, PIN>(gt, gr, A, smem)) return false;
+  } else {
+    if (blockIdx.x == 0) {
+      const MgLevel& Lc = A.lv[N - 1];
+      if (PIN && Lc.g.nn <= FEM_COARSE_WARP_NN) {
+        if (threadIdx.x < 32) mg_coarse_warp<KIND>(A, smem + 128);
         __syncthreads();
       } else {
         mg_coarse<KIND, PIN>(gr, A, smem, cg_r, cg_p, cg_q);
       }
       fem_trace_mark(A.sync, 8);
-      const MgLevel& Lc = A.lv[N - 1];
       if (N == 1) {
         // single level: the coarse solve is the whole preconditioner; r.z pieces
         double a[2] = {0.0, 0.0};
@@ -1089,13 +838,10 @@ __device__ __noinline__ bool mg_vcycle(const GridTeam& gt, const GridReducer& gr
         gr.reduce<2>(a, SL_X(N - 1), smem);
       }
     }
-    if (!tt.sync()) return false;
-    for (int n = b - 1; n >= s; --n)
-      if (!mg_up<KIND, PIN>(tt, gr, A, n, smem)) return false;
-    fem_trace_mark(A.sync, 10);
+    if (!gt.sync()) return false;
   }
-  if (!gt.sync()) return false;
+#pragma unroll 1
   for (int n = s - 1; n >= 0; --n)
-    if (!mg_up<KIND, PIN>(gt, gr, A, n, smem)) return false;
+    if (!mg_up<KIND, PIN, PER>(gt, gr, A, n, smem)) return false;
   return true;
 }

@@ -137,7 +137,7 @@ __device__ __forceinline__ void fem_gather_k(const FemGrid& g, int i, int j, int
 
 // ---------------------------------------------------------------- stencils --
 
-__host__ __device__ __forceinline__ int fem_axis_ncls(int kind, int periodic) {
+__host__ __device__ __forceinline__ constexpr int fem_axis_ncls(int kind, int periodic) {
   if (kind == FEM_Q2_2D) return periodic ? 2 : 4;
   return periodic ? 1 : 3;
 }

@@ -803,17 +803,31 @@ static int mg3_chebyshev(Mg3* M, const G* geo, cudaStream_t s) {
   return FEM_OK;
 }
 
-// In-place Gauss-Jordan inversion of the n x n coarse matrix in M->Ainv
-static int mg3_invert(Mg3* M, int n, cudaStream_t s) {
+int fem_gj_invert(double* A, double* gj, int n, int cap, cudaStream_t s) {
   const long long nn2 = (long long)n * n;
-  const int gb = (int)std::min<long long>((nn2 + 255) / 256, (long long)M->cap * 4);
+  const int gb = (int)std::min<long long>((nn2 + 255) / 256, (long long)cap * 4);
   for (int k = 0; k < n; ++k) {
-    k_mg3_gj_pivot<<<1, 1024, 0, s>>>(n, k, M->Ainv, M->gj, M->gj + n);
-    k_mg3_gj_update<<<gb, 256, 0, s>>>(n, k, M->Ainv, M->gj, M->gj + n);
+    k_mg3_gj_pivot<<<1, 1024, 0, s>>>(n, k, A, gj, gj + n);
+    k_mg3_gj_update<<<gb, 256, 0, s>>>(n, k, A, gj, gj + n);
     if ((k & 255) == 255 || k == n - 1) MG3_TRY(fem_after_launch("k_mg3_gj"));
   }
   MG3_CUDA(cudaStreamSynchronize(s));
   return FEM_OK;
+}
+// In-place inversion of the coarse matrix in M->Ainv
+static int mg3_invert(Mg3* M, int n, cudaStream_t s) { return fem_gj_invert(M->Ainv, M->gj, n, M->cap, s); }
+
+int fem_launch_dense_rows(const FemGrid& g, const double* tab, const uint8_t* pin, double* A, int cap,
+                          cudaStream_t s) {
+  const long long nn2 = (long long)g.nn * g.nn;
+  MG3_CUDA(cudaMemsetAsync(A, 0, sizeof(double) * nn2, s));
+  if (g.kind == FEM_Q1_2D)
+    k_mg2_dense_rows<FEM_Q1_2D><<<mg3_blocks_elem(g.nn, cap), MG3_THREADS, 0, s>>>(g, tab, A);
+  else
+    k_mg2_dense_rows<FEM_Q2_2D><<<mg3_blocks_elem(g.nn, cap), MG3_THREADS, 0, s>>>(g, tab, A);
+  MG3_TRY(fem_after_launch("k_mg2_dense_rows"));
+  k_mg2_dense_fix<<<(int)std::min<long long>((nn2 + 255) / 256, (long long)cap * 4), 256, 0, s>>>(g.nn, pin, 0, 0.0, A);
+  return fem_after_launch("k_mg2_dense_fix");
 }
 
 int mg3_setup(Mg3** out, int nex, int ney, int nez, double lx, double ly, double lz, int nlev,

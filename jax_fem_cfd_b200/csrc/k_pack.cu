@@ -23,12 +23,11 @@
 #include "fem_step_body.cuh"
 
 // dynamic smem (doubles): [0,128) reductions | tiles of the convection apply,
-// the BiCGSTAB operator and the CG phases | CG stencil tables | 1/D of the
-// multigrid levels run inside one CTA
-#define FEM_PACK_SMEM (128 + FEM_CONV_SMEM + FEM_TAB_SMEM + FEM_BLK_SMEM)
+// the BiCGSTAB operator and the CG phases | CG stencil tables (quad4)
+#define FEM_PACK_SMEM (128 + FEM_CONV_SMEM + FEM_MAX_LEVELS * (2 * 81 + 2 * 9))
 static_assert(FEM_CONV_SMEM >= FEM_TILE_SMEM, "the tile region holds the CG tiles too");
 
-template <int KIND>
+template <int KIND, bool PER>
 __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* __restrict__ mem,
                                                               const __grid_constant__ PackParams P) {
   extern __shared__ __align__(128) double smem[];
@@ -36,7 +35,7 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
   __shared__ __align__(16) BiArgs sB;
   __shared__ __align__(16) StepArgs sS;
   __shared__ double sKd[81], sLe[81];
-  __shared__ unsigned int s_round, s_team_round;
+  __shared__ unsigned int s_round;
   constexpr int NEN = KI<KIND>::NEN;
   const int mi = P.idx[blockIdx.y];  // the member this group runs
   const PackStep ps = P.m[mi];
@@ -45,8 +44,7 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
   fem_stage_args(M.C, &sC);
   fem_stage_args(M.B, &sB);
   fem_stage_args(M.S, &sS);
-  fem_tables_to_smem<KIND>(sC, smem + 128 + FEM_CONV_SMEM);
-  fem_block_levels_to_smem(sC, smem + 128 + FEM_CONV_SMEM + FEM_TAB_SMEM);
+  fem_tables_to_smem(sC, smem, 128 + FEM_CONV_SMEM);
   const double theta = 0.5, rho = 1.0, dt = ps.dt, mu = ps.mu;
   // the momentum operator's shared matrix (the solo step's k_lincomb expression)
   const double ka = rho / dt, kb = theta * mu;
@@ -56,7 +54,6 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
   }
   if (threadIdx.x == 0) {
     s_round = 0u;
-    s_team_round = 0u;
     sS.dt = dt;
     sS.mu = mu;
     sS.rho = rho;
@@ -94,7 +91,7 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
     if (threadIdx.x == 0) sC.x = Po;
     if (!gt.sync()) return;
     // 6. pressure MG-PCG (its pinned rows are zeroed after its last barrier)
-    cg_solve<KIND, true>(sC, smem, &s_round, &s_team_round, M.cr, M.cp, M.cq);
+    cg_solve<KIND, true, PER>(sC, smem, &s_round, M.cr, M.cp, M.cq);
     if (!gt.sync()) return;
     // 7. projection and Dirichlet values
     step_ufinal<KIND>(sS, M.Ustar, Po, M.Ud, Uo);
@@ -103,13 +100,14 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
   }
 }
 
-int fem_launch_step_pack(int kind, const PackMember* members, const PackParams& P, int k, int ctas, int blk,
-                         cudaStream_t s) {
+static const void* pack_fn(int periodic) {
+  return periodic ? (const void*)k_step_pack<FEM_Q1_2D, true> : (const void*)k_step_pack<FEM_Q1_2D, false>;
+}
+int fem_launch_step_pack(int kind, int periodic, const PackMember* members, const PackParams& P, int k, int ctas, cudaStream_t s) {
   if (kind != FEM_Q1_2D || k < 1 || k > FEM_PACK_MAX || ctas < 1) return FEM_E_ARG;
-  const void* fn = (const void*)k_step_pack<FEM_Q1_2D>;
-  // the region of the CTA-0 multigrid levels' 1/D only when they run
-  const int dyn = (FEM_PACK_SMEM - (blk ? 0 : FEM_BLK_SMEM)) * (int)sizeof(double);
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, FEM_PACK_SMEM * (int)sizeof(double));
+  const void* fn = pack_fn(periodic);
+  const int dyn = FEM_PACK_SMEM * (int)sizeof(double);
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
   const PackMember* m = members;
   PackParams p = P;
   void* args[] = {&m, &p};
@@ -128,9 +126,13 @@ int fem_launch_step_pack(int kind, const PackMember* members, const PackParams& 
 }
 
 int fem_pack_occupancy(int* per_sm) {
-  const void* fn = (const void*)k_step_pack<FEM_Q1_2D>;
+  *per_sm = 1 << 30;
   const int dyn = FEM_PACK_SMEM * (int)sizeof(double);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess) return -1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, FEM_THREADS, dyn) != cudaSuccess) return -1;
+  for (int per = 0; per < 2; ++per) {
+    int a = 0;
+    if (cudaFuncSetAttribute(pack_fn(per), cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess) return -1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, pack_fn(per), FEM_THREADS, dyn) != cudaSuccess) return -1;
+    *per_sm = a < *per_sm ? a : *per_sm;
+  }
   return 0;
 }
