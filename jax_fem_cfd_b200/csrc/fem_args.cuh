@@ -31,6 +31,7 @@ struct BiArgs {
   const double* cvf;
   double cv_coef;
   FemQuadTab qt;
+  FemConv3 c3;  // hex8, if c3.U is set: the whole operator, applied from the nodal velocities (fem_conv3.cuh)
 };
 
 struct StepArgs {
@@ -150,12 +151,8 @@ int fem_launch_conv_vjp(const FemGrid& g, const FemQuadTab& qt, int ncomp, const
 int fem_launch_transport_vjp(const FemGrid& g, const FemQuadTab& qt, const double* Un, const double* U,
                              const double* lam, const double* phin, const double* phi, double dt, double D, int supg,
                              double* gen, double* geu, double* yn, double* yu, cudaStream_t s);
-// hex8: the Gauss-point factors (32 per element, element-major) and
-// y = alpha Ash x + cc Ce x per component (3 components) from them
-int fem_launch_conv_factors3(const FemGrid& g, const FemQuadTab& qt, const double* U, double bd, double* fq,
-                             cudaStream_t s);
-int fem_launch_conv_apply3(const FemGrid& g, const FemQuadTab& qt, const double* fq, double cc, double alpha,
-                           const double* Ash, const double* x, double* y, int grid, int* err, cudaStream_t s);
+// hex8: y = (mass Me + diff Le + cc Ce(U)) x for 3 components (fem_conv3.cuh)
+int fem_launch_conv_apply3(const FemGrid& g, const FemConv3& op, const double* x, double* y, int grid, cudaStream_t s);
 
 // hex8, 3 components: y = (alpha A + beta B_e) x, element-centric (B per element, not transposed, no C)
 int fem_launch_ebe3e(const FemGrid& g, const MatCombo& m, const double* x, double* y, int grid, cudaStream_t s);

@@ -3,37 +3,35 @@
 #include "fem_b200.h"
 #include "fem_args.cuh"
 
-template <int KIND, int NC, class Src>
-__device__ __forceinline__ void bi_apply(const BiArgs& A, const MatCombo& op, int i, const Src& src, double (&y)[NC]) {
-  int ix, iy, iz;
-  fem_ij(A.g, i, ix, iy, iz);
-  fem_gather_k<KIND, NC>(A.g, ix, iy, iz, op, src, y);
-  if (A.mask) {
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-      if (A.mask[i + (size_t)c * A.g.nn]) y[c] = src(i, c);
-  }
-}
-
 // The operator apply of the solver: the element-by-element product of op on
-// load(j, c), or (OTF) op.alpha op.A + cv_coef Ce from Gauss-point factors on
-// comb of the staged sources (Ce never materialised).
-template <int KIND, int NC, bool OTF, int NSRC, class Team, class Load, class Comb, class Body>
+// load(j, c), or (OTF) on comb of the staged sources with Ce never materialised:
+// op.alpha op.A + cv_coef Ce from Gauss-point factors (2D), c3 (hex8). Identity
+// rows where A.mask is set; body(i, y, x, a) with a = aux (null: unused) at node i.
+template <int KIND, int NC, bool OTF, bool AUX, int NSRC, class Team, class Load, class Comb, class Body>
 __device__ __forceinline__ void bi_tiled_apply(const Team& tm, const BiArgs& A, const MatCombo& op, double* tsm,
-                                               const FemC3Tma& tma, const Load& load,
-                                               const double* const (&src)[NSRC], const Comb& comb,
-                                               const Body& body) {
+                                               const Load& load, const double* const (&src)[NSRC], const Comb& comb,
+                                               const double* aux, const Body& body) {
+  auto row = [&](int i, const double(&y)[NC], const double(&x)[NC]) {
+    double v[NC], a[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const size_t o = i + c * (size_t)A.g.nn;
+      v[c] = (A.mask && A.mask[o]) ? x[c] : y[c];
+      a[c] = AUX ? aux[o] : 0.0;
+    }
+    body(i, v, x, a);
+  };
   if constexpr (OTF && KIND == FEM_HEX8) {
-    fem_tiled_conv3<NC, NSRC>(tm, A.g, tsm, tma, src, comb, A.cvf, A.qt, A.cv_coef, op.alpha, op.A, body);
+    fem_march_conv3<NSRC, AUX>(tm, A.g, tsm, src, comb, A.c3, A.mask, aux, body);
   } else if constexpr (OTF) {
-    fem_tiled_conv<KIND, NC, NSRC>(tm, A.g, tsm, src, comb, A.cvf, A.qt, A.cv_coef, op.alpha, op.A, body);
+    fem_tiled_conv<KIND, NC, NSRC>(tm, A.g, tsm, src, comb, A.cvf, A.qt, A.cv_coef, op.alpha, op.A, row);
   } else if constexpr (KIND == FEM_HEX8) {
     // explicit per-element matrices: element-centric (fem_tiled_ebe3e); other
     // combinations (transposed B, a third matrix) node-centric
-    if (op.B && !op.transB && !op.C) fem_tiled_ebe3e<NC>(tm, A.g, tsm, load, op, body);
-    else fem_tiled_ebe<KIND, NC>(tm, A.g, tsm, load, op, body);
+    if (op.B && !op.transB && !op.C) fem_tiled_ebe3e<NC>(tm, A.g, tsm, load, op, row);
+    else fem_tiled_ebe<KIND, NC>(tm, A.g, tsm, load, op, row);
   } else {
-    fem_tiled_ebe<KIND, NC>(tm, A.g, tsm, load, op, body);
+    fem_tiled_ebe<KIND, NC>(tm, A.g, tsm, load, op, row);
   }
 }
 
@@ -43,7 +41,7 @@ __device__ __forceinline__ void bi_tiled_apply(const Team& tm, const BiArgs& A, 
 // operator's staging; s_round: the CTA's completed barriers on A.sync's counter.
 template <int KIND, int NC, bool OTF>
 __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& op, double* smem, double* tsm,
-                                               const FemC3Tma& tma, unsigned int* s_round) {
+                                               unsigned int* s_round) {
   const GridTeam gt = GridTeam::grid(&A.sync, s_round);
   const GridReducer gr{&A.sync};
   const int nn = A.g.nn;
@@ -56,14 +54,14 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
     {
       double a[2] = {0.0, 0.0};
       const double* sx0[1] = {A.x};
-      bi_tiled_apply<KIND, NC, OTF>(gt, A, op, tsm, tma, [&](int j, int c) { return A.x[j + c * N]; }, sx0,
-                                    [](int, const double(&v)[1]) { return v[0]; },
-                              [&](int i, const double(&Ax)[NC], const double(&xc)[NC]) {
+      bi_tiled_apply<KIND, NC, OTF, true>(gt, A, op, tsm, [&](int j, int c) { return A.x[j + c * N]; }, sx0,
+                                          [](int, const double(&v)[1]) { return v[0]; }, A.b,
+                                          [&](int i, const double(&Ax)[NC], const double(&)[NC],
+                                              const double(&bv)[NC]) {
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           const size_t o = i + c * N;
-          const double ax = (A.mask && A.mask[o]) ? xc[c] : Ax[c];
-          const double bi = A.b[o], ri = bi - ax;
+          const double bi = bv[c], ri = bi - Ax[c];
           A.r[o] = ri;
           A.rhat[o] = ri;
           A.p0[o] = ri;
@@ -99,16 +97,16 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
         };
         double a[1] = {0.0};
         const double* spn[3] = {r, pold, qold};
-        bi_tiled_apply<KIND, NC, OTF>(gt, A, op, tsm, tma, pn, spn,
-                                      [&](int, const double(&v)[3]) { return v[0] + beta * (v[1] - omega * v[2]); },
-                                      [&](int i, const double(&qv)[NC], const double(&pc)[NC]) {
+        bi_tiled_apply<KIND, NC, OTF, true>(gt, A, op, tsm, pn, spn,
+                                            [&](int, const double(&v)[3]) { return v[0] + beta * (v[1] - omega * v[2]); },
+                                            A.rhat, [&](int i, const double(&q)[NC], const double(&pc)[NC],
+                                                        const double(&rh)[NC]) {
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
             const size_t o = i + c * N;
-            const double q = (A.mask && A.mask[o]) ? pc[c] : qv[c];
             pnew[o] = pc[c];
-            qnew[o] = q;
-            a[0] += A.rhat[o] * q;
+            qnew[o] = q[c];
+            a[0] += rh[c] * q[c];
           }
         });
         gr.reduce<1>(a, SL_BI + 1, smem);
@@ -124,17 +122,16 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
       {
         double a[3] = {0.0, 0.0, 0.0};
         const double* ssv[2] = {r, qnew};
-        bi_tiled_apply<KIND, NC, OTF>(gt, A, op, tsm, tma, sv, ssv,
-                                      [&](int, const double(&v)[2]) { return v[0] - alpha_ * v[1]; }, [&](int i, const double(&tvv)[NC], const double(&sc)[NC]) {
+        bi_tiled_apply<KIND, NC, OTF, false>(gt, A, op, tsm, sv, ssv,
+                                             [&](int, const double(&v)[2]) { return v[0] - alpha_ * v[1]; }, nullptr,
+                                             [&](int i, const double(&tv)[NC], const double(&sc)[NC],
+                                                 const double(&)[NC]) {
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
-            const size_t o = i + c * N;
-            const double tvc = (A.mask && A.mask[o]) ? sc[c] : tvv[c];
-            const double s = sc[c];
-            A.t[o] = tvc;
-            a[0] += s * s;
-            a[1] += tvc * s;
-            a[2] += tvc * tvc;
+            A.t[i + c * N] = tv[c];
+            a[0] += sc[c] * sc[c];
+            a[1] += tv[c] * sc[c];
+            a[2] += tv[c] * tv[c];
           }
         });
         gr.reduce<3>(a, SL_BI + 2, smem);
@@ -147,22 +144,26 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
       {
         double a[2] = {0.0, 0.0};
         for (int i = gt.rank(); i < nn; i += gt.size()) {
+          // every load before the first store, which the compiler cannot move loads across
+          double s[NC], xv[NC], pv[NC], tv[NC], rh[NC];
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
             const size_t o = i + c * N;
-            const double s = sv(i, c);
-            double xn, rn;
-            if (exit_early) {
-              xn = A.x[o] + alpha_ * pnew[o];
-              rn = s;
-            } else {
-              xn = A.x[o] + (alpha_ * pnew[o] + omega_ * s);
-              rn = s - omega_ * A.t[o];
-            }
+            s[c] = sv(i, c);
+            xv[c] = A.x[o];
+            pv[c] = pnew[o];
+            tv[c] = A.t[o];
+            rh[c] = A.rhat[o];
+          }
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const size_t o = i + c * N;
+            const double xn = exit_early ? xv[c] + alpha_ * pv[c] : xv[c] + (alpha_ * pv[c] + omega_ * s[c]);
+            const double rn = exit_early ? s[c] : s[c] - omega_ * tv[c];
             A.x[o] = xn;
             A.r[o] = rn;
             a[0] += rn * rn;
-            a[1] += A.rhat[o] * rn;
+            a[1] += rh[c] * rn;
           }
         }
         gr.reduce<2>(a, SL_RR, smem);  // SL_RR, SL_RSUM (= rhat.r)

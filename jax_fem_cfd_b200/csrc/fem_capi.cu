@@ -477,7 +477,7 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   FEM_ALLOC(c->Ce, (size_t)g.ne * per);
   FEM_ALLOC(c->vcv, vn);
   FEM_ALLOC(c->ebe_tab, FEM_TAB_MAX);
-  FEM_ALLOC(c->cvf, g.kind == FEM_HEX8 ? (size_t)FEM_C3_NF * g.ne : (size_t)3 * c->nq * g.ne);
+  if (g.kind != FEM_HEX8) FEM_ALLOC(c->cvf, (size_t)3 * c->nq * g.ne);
   FEM_ALLOC(c->dotpart, 4096);
   cudaStream_t s = 0;
   FEM_CHECK(cudaMemset(c->bar, 0, sizeof(unsigned int)));
@@ -537,12 +537,9 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
         c->qt.dz[q][b] = nd == 3 ? hdN[(q * nd + 2) * nen + b] : 0.0;
       }
     }
-    // on the fly by default in 2D; hex8 keeps the explicit Ce unless asked
-    // (FEM_CONV_OTF=1): on the 256 x 64 x 64 channel the explicit form ran
-    // 96.2 steps/s against 83.4, its 64 coefficients per element costing less
-    // than the on-the-fly element rows (~5x the FP64 work of a Ce row product)
+    // on the fly unless FEM_CONV_OTF=0
     const char* ev = getenv("FEM_CONV_OTF");
-    c->conv_otf = ev ? (atoi(ev) != 0) : (g.kind != FEM_HEX8);
+    c->conv_otf = ev ? (atoi(ev) != 0) : 1;
     // Q2: the tensor factors of the on-the-fly operator; without them (a table
     // that does not factor) fem_step4 builds Ce explicitly
     if (g.kind == FEM_Q2_2D && !q2_tensor_factors(c->qt)) c->conv_otf = 0;
@@ -1055,7 +1052,7 @@ extern "C" int fem_mg_vcycle(fem_ctx* c, const double* r, double* z, cudaStream_
 
 static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t* mask, const double* b, double* x,
                         double tol, double atol, int maxiter, int* iters, int* status, cudaStream_t s,
-                        const double* cvf = nullptr, double cv_coef = 0.0) {
+                        const double* cvf = nullptr, double cv_coef = 0.0, const FemConv3* c3 = nullptr) {
   if (ncomp < 1 || ncomp > c->ndim) return FEM_E_ARG;  // workspace holds ndim*nn per vector
   BiArgs A;
   memset(&A, 0, sizeof(A));
@@ -1080,8 +1077,10 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
   A.cvf = cvf;
   A.cv_coef = cv_coef;
   A.qt = c->qt;
+  if (c3) A.c3 = *c3;
   FEM_TRY(reset_sync(c, s));
-  A.sync.ncols = ctx_grid_for(c);
+  // the hex8 march splits to single planes
+  A.sync.ncols = c3 ? (int)std::min<long long>(c->max_coop, fem_c3_units(c->g)) : ctx_grid_for(c);
   return fem_launch_bicgstab(ncomp, A, A.sync.ncols, s);
 }
 
@@ -1111,10 +1110,10 @@ extern "C" int fem_step4(fem_ctx* c, const double* Un, const double* Pn, double 
   // 1. Ce(U_n), beta = 1/2 (solvers/standard.py:152). On the fly: Ce is never
   // built; its Gauss-point factors are, and (mu Le + rho Ce) U_n of the momentum
   // rhs is applied here.
-  const bool otf = c->conv_otf && c->cvf;
+  const bool otf = c->conv_otf && (c->cvf || g.kind == FEM_HEX8);
+  const double hx = c->lx / g.nex, hy = c->ly / g.ney, hz = g.kind == FEM_HEX8 ? c->lz / g.nez : 0.0;  // of a hex8 box
   if (otf && g.kind == FEM_HEX8) {
-    FEM_TRY(fem_launch_conv_factors3(g, c->qt, Un, 0.5, c->cvf, s));
-    FEM_TRY(fem_launch_conv_apply3(g, c->qt, c->cvf, rho, mu, c->Le, Un, c->vcv, c->sms, c->err, s));
+    FEM_TRY(fem_launch_conv_apply3(g, fem_conv3_coef(Un, hx, hy, hz, rho, 0.5, 0.0, mu), Un, c->vcv, c->sms, s));
   } else if (otf) {
     FEM_TRY(fem_launch_conv_factors(g, c->qt, Un, 0.5, c->cvf, s));
     FEM_TRY(fem_launch_conv_apply(2, g, c->qt, c->cvf, rho, mu, c->Le, Un, c->vcv, c->sms, s));
@@ -1153,6 +1152,10 @@ extern "C" int fem_step4(fem_ctx* c, const double* Un, const double* Pn, double 
     if (!c->mixmom) FEM_TRY(mixmom_create(&c->mixmom, g, nd, c->nq, c->sms));
     FEM_TRY(mixmom_solve(c->mixmom, c->qt, c->cvf, c->Kd, theta * rho, S.dmask, c->rhsU, c->Uhat, tol,
                          FEM_MIXED_MOMENTUM_INNER, c->mx_cycles, iters, status, c->sms, s, c->cap_stream));
+  } else if (otf && g.kind == FEM_HEX8) {
+    const FemConv3 op = fem_conv3_coef(Un, hx, hy, hz, theta * rho, 0.5, rho / dt, theta * mu);
+    FEM_TRY(run_bicgstab(c, nd, MatCombo{}, S.dmask, c->rhsU, c->Uhat, tol, 0.0, 0, iters, status, s, nullptr, 0.0,
+                         &op));
   } else if (otf) {
     const MatCombo op{c->Kd, 1.0, nullptr, 0.0, 0, nullptr, 0.0};
     FEM_TRY(run_bicgstab(c, nd, op, S.dmask, c->rhsU, c->Uhat, tol, 0.0, 0, iters, status, s, c->cvf, theta * rho));

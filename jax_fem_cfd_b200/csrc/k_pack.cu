@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
   }
   __syncthreads();
   const MatCombo op{sKd, 1.0, nullptr, 0.0, 0, nullptr, 0.0};
-  const FemC3Tma tma{nullptr, nullptr, sC.sync.err};  // 2D: no TMA factor copies
   const GridTeam gt = GridTeam::grid(&sC.sync, &s_round);
   const size_t nn = sS.g.nn;
   int* stat = M.stat;
@@ -82,7 +81,7 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
     step_mom_rhs<KIND>(sS, Un, Pn, M.Ud, nullptr, M.rhsU, M.Uhat, M.gPn);
     if (!gt.sync()) return;
     // 3. momentum BiCGSTAB (ends on a barrier)
-    bicgstab_solve<KIND, 2, true>(sB, op, smem, smem + 128, tma, &s_round);
+    bicgstab_solve<KIND, 2, true>(sB, op, smem, smem + 128, &s_round);
     // 4. U*
     step_ustar((int)(2 * nn), dt / rho, M.Uhat, M.gPn, sS.M, M.Ustar);
     if (!gt.sync()) return;
