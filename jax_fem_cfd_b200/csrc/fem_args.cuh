@@ -6,7 +6,7 @@
 #include "fem_conv3.cuh"
 
 #define FEM_THREADS 512
-#define FEM_CG_THREADS 256  // 2D k_cg / k_vcycle
+#define FEM_CG_THREADS 256  // k_cg / k_vcycle
 #define FEM_OP_THREADS 256
 // dynamic smem of k_cg / k_vcycle (doubles): reduction scratch, tile staging, the
 // levels' tables; at most 14 levels of 16 classes x 25 coefficients twice

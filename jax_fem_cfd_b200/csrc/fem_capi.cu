@@ -228,11 +228,11 @@ static int dense_level(const fem_ctx* c, const double** C, int* ld) {
 // ctx_grid_for CTAs of 16 warps, at most one round of the whole device.
 static int cg_items(const fem_ctx* c) { return std::min(ctx_grid_for(c) * 16, c->sms * (FEM_CG_THREADS / 32)); }
 
-// CTAs of a CG solve. 2D: one warp of work per CTA while there are items (a warp
+// CTAs of a CG solve: one warp of work per CTA while there are items (a warp
 // alone on its SM runs fastest: 64^2 quad4 cavity step on 9 CTAs 541 us, on 145
 // 373 us), and enough for the dense level's rows.
 static int cg_grid_for(const fem_ctx* c) {
-  if (c->g.kind == FEM_HEX8) return ctx_grid_for(c);
+  if (c->g.kind == FEM_HEX8) return (int)std::min<long long>(c->max_coop, fem_l3_units(c->g));
   if (cg_by_items(c)) return std::min(cg_items(c), c->max_coop);
   const double* C;
   int ld;

@@ -37,22 +37,22 @@ __device__ __forceinline__ bool cg_apply_prec(const GridTeam& gt, const GridRedu
     const double* __restrict__ D = L0.diag;
     const double* __restrict__ iD = L0.invD;
     const double* src1[2] = {r, iD};
-    fem_tiled_stencil<KIND, 2>(gt, L0.g, L0.tab, smem + 128, src1,
-                               [](int, const double(&v)[2]) { return v[0] * v[1]; },
-                               [&](int i, int, int, int, double v, double) {
-                                 double d1l = v / D[i];
-                                 if (ap && ap[i]) d1l = pt ? r[i] / D[i] : 0.0;
-                                 T[i] = d1l;
-                               });
+    const double* const aux[2] = {D, r};
+    fem_lattice3<2, 2>(gt, L0.g, L0.tab, src1, ap, aux, [](const double(&v)[2]) { return v[0] * v[1]; },
+                       [&](int i, double v, double, bool flag, const double(&x)[2]) {
+                         T[i] = flag ? (pt ? x[1] / x[0] : 0.0) : v / x[0];
+                       },
+                       FemNoHook());
     if (!gt.sync()) return false;
     const double* src2[1] = {T};
-    fem_tiled_stencil<KIND, 1>(gt, L0.g, L0.tab, smem + 128, src2, [](int, const double(&v)[1]) { return v[0]; },
-                               [&](int i, int, int, int, double t, double) {
-                                 if (ap && ap[i]) t = pt ? T[i] : 0.0;
-                                 const double zi = 3 * (r[i] / D[i]) - 3 * T[i] + t / D[i];
-                                 zo[i] = zi;
-                                 acc[0] += r[i] * zi;
-                               });
+    fem_lattice3<1, 2>(gt, L0.g, L0.tab, src2, ap, aux, [](const double(&v)[1]) { return v[0]; },
+                       [&](int i, double t, double Ti, bool flag, const double(&x)[2]) {
+                         if (flag) t = pt ? Ti : 0.0;
+                         const double zi = 3 * (x[1] / x[0]) - 3 * Ti + t / x[0];
+                         zo[i] = zi;
+                         acc[0] += x[1] * zi;
+                       },
+                       FemNoHook());
   } else {
     const FemGrid& g = L0.g;
     constexpr int nc = fem_axis_ncls(KIND, PER), S1 = 256 * KS<KIND>::NC;  // S1: from source to source in a slot
@@ -150,10 +150,13 @@ __device__ __forceinline__ bool cg_residual(const GridTeam& gt, const GridReduce
   };
   if constexpr (KIND == FEM_HEX8) {
     const double* srcx[1] = {A.x};
-    fem_tiled_stencil<KIND, 1>(gt, g, L0.tab, smem + 128, srcx, [](int, const double(&v)[1]) { return v[0]; },
-                               [&](int i, int, int, int, double Ax, double) {
-                                 body(i, (pin0 && pin0[i]) ? 0.0 : Ax, b[i] - bm, L0.invD[i]);
-                               });
+    const double* const aux[3] = {b, L0.invD, L0.diag};
+    fem_lattice3<1, 3>(gt, g, L0.tab, srcx, pin0, aux, [](const double(&v)[1]) { return v[0]; },
+                       [&](int i, double Ax, double, bool flag, const double(&v)[3]) {
+                         body(i, flag ? 0.0 : Ax, v[0] - bm, v[1]);
+                         if (A.prec == FEM_PREC_JACOBI) A.z[i] = ro[i] / v[2];
+                       },
+                       FemNoHook());
   } else {
     const double* __restrict__ x0 = A.x;
     constexpr int nc = fem_axis_ncls(KIND, PER), S1 = 256 * KS<KIND>::NC;  // S1: from source to source in a slot
@@ -224,12 +227,13 @@ __device__ __forceinline__ bool cg_direction(const GridTeam& gt, const GridReduc
     a[0] += pn * q;
   };
   if constexpr (KIND == FEM_HEX8) {
-    const double* src[3] = {s0, s1, s2};
-    fem_tiled_stencil<KIND, 3>(gt, g, L0.tab, smem + 128, src, [&](int, const double(&v)[3]) { return comb(v); },
-                               [&](int i, int, int, int, double q, double pn) {
-                                 body(i, (pin0 && pin0[i]) ? 0.0 : q, pn);
-                               },
-                               pre);
+    // Jacobi: z = r / D was left by the last phase that wrote r; the first p has no predecessor
+    const double* src[2] = {prec == FEM_PREC_NONE ? A.r : A.z, have_p ? pold : A.r};
+    const double* const aux[1] = {nullptr};
+    fem_lattice3<2, 1>(gt, g, L0.tab, src, pin0, aux,
+                       [&](const double(&v)[2]) { return have_p ? v[0] + be * v[1] : v[0]; },
+                       [&](int i, double q, double pn, bool flag, const double(&)[1]) { body(i, flag ? 0.0 : q, pn); },
+                       pre);
   } else {
     constexpr int nc = fem_axis_ncls(KIND, PER), S1 = 256 * KS<KIND>::NC;  // S1: from source to source in a slot
     const double* dt = smem + L0.tab_s + 2 * fem_tab_doubles(g) + fem_stencil_ncls(g);
@@ -268,9 +272,11 @@ __device__ __forceinline__ bool cg_update(const GridTeam& gt, const GridReducer&
   const double* __restrict__ Ap = A.Ap;
   const double* __restrict__ iD0 = A.lv[0].invD;
   const bool sums_d = !PIN || A.prec != FEM_PREC_MG;
+  // hex8 Jacobi leaves z = r / D: phase A reads each node's z several times
+  const bool put_z = KIND == FEM_HEX8 && A.prec == FEM_PREC_JACOBI;
   auto span = [&](int first, int end, int stride) {
     for (int i0 = first; i0 < end; i0 += U * stride) {
-      double xv[U], pv[U], rv[U], av[U], iv[U];
+      double xv[U], pv[U], rv[U], av[U], iv[U], dv[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int i = i0 + u * stride;
@@ -280,6 +286,7 @@ __device__ __forceinline__ bool cg_update(const GridTeam& gt, const GridReducer&
           rv[u] = r[i];
           av[u] = Ap[i];
           iv[u] = sums_d ? iD0[i] : 0.0;
+          dv[u] = put_z ? A.lv[0].diag[i] : 1.0;
         }
       }
 #pragma unroll
@@ -289,6 +296,7 @@ __device__ __forceinline__ bool cg_update(const GridTeam& gt, const GridReducer&
           x[i] = xv[u] + alpha * pv[u];
           const double ri = rv[u] - alpha * av[u];
           r[i] = ri;
+          if (put_z) A.z[i] = ri / dv[u];
           a4[0] += ri * ri;
           a4[1] += ri;
           a4[2] += ri * iv[u];

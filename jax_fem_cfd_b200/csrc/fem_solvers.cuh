@@ -15,6 +15,7 @@
 #include "fem_ops.cuh"
 #include "fem_stencil.cuh"
 #include "fem_strip.cuh"
+#include "fem_lattice3.cuh"
 
 #define FEM_MAX_LEVELS 14
 

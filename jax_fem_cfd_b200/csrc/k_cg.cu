@@ -3,7 +3,7 @@
 
 
 template <int KIND, bool PIN, bool PER>
-__global__ void __launch_bounds__(KIND == FEM_HEX8 ? FEM_THREADS : FEM_CG_THREADS, 1) k_cg(CgArgs Aparam, double* cg_r, double* cg_p, double* cg_q) {
+__global__ void __launch_bounds__(FEM_CG_THREADS, 1) k_cg(CgArgs Aparam, double* cg_r, double* cg_p, double* cg_q) {
   // [0,128) reductions, [128, +FEM_TILE_SMEM) tiles, then the stencil tables
   extern __shared__ __align__(16) double smem[];
   __shared__ __align__(16) CgArgs sA;
@@ -57,7 +57,6 @@ __global__ void __launch_bounds__(FEM_CG_THREADS, 1) k_vcycle(CgArgs Aparam, dou
   for (int i = gt.rank(); i < nn; i += gt.size()) z[i] = L0.t[i] - mz;
 }
 
-static int threads_of(int kind) { return kind == FEM_HEX8 ? FEM_THREADS : FEM_CG_THREADS; }
 static int coop_launch(const void* fn, int grid, int threads, void** args, cudaStream_t s, const char* what,
                        size_t dyn) {
   cudaLaunchConfig_t cfg = {};
@@ -101,7 +100,7 @@ int fem_launch_cg(const CgArgs& A, int grid, double* cr, double* cp, double* cq,
   void* args[] = {&a, &cr, &cp, &cq};
   const FemGrid& g = A.lv[0].g;
   const int kind = g.kind;
-  return coop_launch(cg_fn(kind, A.pinned, g.periodic), grid, threads_of(kind), args, s, "k_cg", cg_dyn_smem(A));
+  return coop_launch(cg_fn(kind, A.pinned, g.periodic), grid, FEM_CG_THREADS, args, s, "k_cg", cg_dyn_smem(A));
 }
 int fem_launch_vcycle(const CgArgs& A, int grid, double* cr, double* cp, double* cq, double* z, cudaStream_t s) {
   CgArgs a = A;
@@ -119,7 +118,7 @@ int fem_coop_occupancy_cg(int* occ) {
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, FEM_DYN_SMEM_MAX) != cudaSuccess)
           return -1;
         int a = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fn, threads_of(kind), FEM_DYN_SMEM_MAX) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fn, FEM_CG_THREADS, FEM_DYN_SMEM_MAX) != cudaSuccess)
           return -1;
         m = a < m ? a : m;
       }

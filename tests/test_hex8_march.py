@@ -35,3 +35,44 @@ def test_step_from_nodal_velocities(nex, ney, nez, ctas, monkeypatch):
         out.append((Uo.cpu().numpy(), Po.cpu().numpy()))
     for a, b in zip(*out):
         assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("ctas", [0, 1, 5])
+@pytest.mark.parametrize("precond", ["jacobi", "approx_inv", None])
+@pytest.mark.parametrize("nex,ney,nez", [(1, 1, 1), (29, 2, 1), (30, 3, 2), (59, 4, 3), (60, 5, 7)])
+def test_cg_two_iterations(nex, ney, nez, precond, ctas):
+    """Two CG iterations where the warps' columns of 30 x 2 nodes and runs of planes
+    end, against the oracle's CG. Sums of at most 27 terms, two iterations: 1e-11."""
+    from jax_fem_cfd_b200 import _lib
+    from jax_fem_cfd_b200.context import Context, Mesh, make_mask, ptr, stream
+    from oracle import element as oel, emult as oem, mesh as om, shape as osh, solvers as osv
+    box = (2.0, 1.5, 0.7)
+    ctx = Context(Mesh(2, False, nex, ney, nez, *box))
+    ctx.set_bc(None, make_mask(np.array([0]), ctx.nn), True)
+    _lib.call("fem_ctx_set_max_ctas", ctx.handle, ctas, None)
+    nc, nconn, *_ = om.create_mesh_3d(nex, ney, nez, *box)
+    wq, _, dN = osh.hex8_shape_functions(nc[nconn[0]])
+    Le = oel.laplacian_element_calc(wq, dN)
+    D = oel.laplacian_diag(Le, nconn, ctx.nn)
+    b = np.random.default_rng(ctx.nn).standard_normal(ctx.nn)
+    b[0] = 0.0
+
+    def lhs(v):
+        y = oem.laplacian_element_mult(v, Le, nconn, ctx.nn)
+        y[0] = 0.0
+        return y
+
+    def approx(r):  # solvers/standard.py:225-234
+        t = lhs(r / D) / D
+        return 3 * (r / D) - 3 * t + lhs(t) / D
+
+    M = {"jacobi": lambda r: r / D, "approx_inv": approx, None: None}[precond]
+    xo, _ = osv.cg(lhs, b, x0=np.zeros_like(b), tol=1e-30, maxiter=2, M=M)
+    xo[0] = 0.0
+    r = torch.as_tensor(b, device="cuda")
+    x = torch.zeros_like(r)
+    it = torch.zeros(2, dtype=torch.int32, device="cuda")
+    _lib.call("fem_pressure_solve", ctx.handle, ptr(r), ptr(x), 1e-30, 0.0, 2, _lib.PREC[precond], 0, 1, ptr(it),
+              ptr(it[1:]), stream())
+    assert int(it[0]) == 2
+    assert np.linalg.norm(x.cpu().numpy() - xo) <= 1e-11 * np.linalg.norm(xo)
