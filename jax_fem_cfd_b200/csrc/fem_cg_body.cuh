@@ -5,8 +5,8 @@
 // Preconditioner application z = M r and gamma = r . z; after a V-cycle gamma and
 // the mean of z are left to the next phase (deferred).
 template <int KIND, bool PIN, bool PER>
-__device__ __forceinline__ bool cg_apply_prec(const GridTeam& gt, const GridReducer& gr, const CgArgs& A, double* smem,
-                                              double* cg_r, double* cg_p, double* cg_q, double rr, double r2d,
+__device__ __forceinline__ bool cg_apply_prec(const GridTeam& gt, const GridReducer& gr, const CgArgs& A,
+                                              CgResidual& r0, double* smem, double* cg_r, double* cg_p, double* cg_q, double rr, double r2d,
                                               double& gamma, double& mz, bool& deferred) {
   const MgLevel& L0 = A.lv[0];
   mz = 0.0;
@@ -20,14 +20,14 @@ __device__ __forceinline__ bool cg_apply_prec(const GridTeam& gt, const GridRedu
     return true;
   }
   if constexpr (KIND != FEM_HEX8) if (A.prec == FEM_PREC_MG) {
-    if (!mg_vcycle<KIND, PIN, PER>(gt, gr, A, smem, cg_r, cg_p, cg_q)) return false;
+    if (!mg_vcycle<KIND, PIN, PER>(gt, gr, A, r0, smem, cg_r, cg_p, cg_q)) return false;
     deferred = true;  // the next phase A reads gamma and mz (cg_mg_from)
     return true;
   }
   // approximate inverse: 2-term Neumann series (T = D^-1 L D^-1 r, then
   // z = 3 D^-1 r - 3 T + D^-1 L T)
   const bool pt = (A.prec == FEM_PREC_APPROX_INV_PT);
-  const double* __restrict__ r = A.r;
+  const double* r = r0.now();
   const uint8_t* __restrict__ ap = A.ai_pin;
   double* __restrict__ T = L0.t;
   double* __restrict__ zo = A.z;
@@ -62,15 +62,21 @@ __device__ __forceinline__ bool cg_apply_prec(const GridTeam& gt, const GridRedu
       return fem_axis_cls(KIND, PER, ry, g.ney) * nc + fem_axis_cls(KIND, PER, gx, g.nex);
     };
     // ai_pin is always a mask of the context (whole words)
-    fem_strip_lattice<KIND, PER, 2, 2>(
+    const double* __restrict__ rf = r0.from();
+    const bool upd = r0.update;
+    double arr[1] = {0.0};
+    const int slm[1] = {SL_RM};
+    fem_strip_lattice<KIND, PER, 3, 2>(
         gt, g, L0.pl, smem + L0.tab_s, smem + 128,
         [&](int i, unsigned slot) {
-          fem_ring_copy(slot, r + i);
+          fem_ring_copy(slot, rf + i);
           fem_ring_copy_mask(slot + S1, ap, i);
+          if (upd) fem_ring_copy(slot + 2 * S1, r0.Ap + i);
         },
         [&](int ry, int gx, int i, unsigned slot, double(&car)[2], bool& flag) {
           const int k = cls(ry, gx);
-          const double ri = fem_ring_get(slot);
+          double ri = fem_ring_get(slot);
+          if (upd) ri -= r0.alpha * fem_ring_get(slot + 2 * S1);
           car[0] = ri;
           car[1] = dt[k];
           flag = fem_ring_byte(slot + S1, i);
@@ -78,9 +84,21 @@ __device__ __forceinline__ bool cg_apply_prec(const GridTeam& gt, const GridRedu
         },
         [&](int i, double v, const double(&car)[2], bool flag) {
           T[i] = flag ? (pt ? car[0] / car[1] : 0.0) : v / car[1];
+          if (upd) {
+            r0.out[i] = car[0];
+            arr[0] += car[0] * car[0];
+          }
         },
-        [](int) {}, FemNoHook());
-    if (!gt.sync()) return false;
+        [&](int it) {
+          if (upd) gr.item_sums<fem_items<KIND, PIN>(), 1>(arr, slm, it);
+        },
+        FemNoHook());
+    if (upd) {
+      if (!gr.finish_items<fem_items<KIND, PIN>(), 1>(gt, arr, slm, smem)) return false;
+      if (!r0.go_on(gr, smem)) return true;
+    } else if (!gt.sync()) {
+      return false;
+    }
     fem_strip_lattice<KIND, PER, 3, 3>(
         gt, g, L0.pl, smem + L0.tab_s, smem + 128,
         [&](int i, unsigned slot) {
@@ -183,10 +201,13 @@ __device__ __forceinline__ bool cg_residual(const GridTeam& gt, const GridReduce
 // Phase A: p = z + beta p_old (z the preconditioned residual: r, r / D, z or the
 // V-cycle's z minus its mean), A p and p.Ap. With `pending` the V-cycle's sums are
 // read here (beta, gamma and mz are set), their loads overlapping the first rows'.
+// 2D: x += alpha p_old as well, the last iteration's step (the update would read p
+// once more for it); the copies of x at halo nodes, which their owners may be
+// writing, are not used.
 template <int KIND, bool PIN, bool PER>
 __device__ __forceinline__ bool cg_direction(const GridTeam& gt, const GridReducer& gr, const CgArgs& A, double* smem,
-                                          int cur, bool have_p, bool pending, double& beta, double& gamma,
-                                             double& mz) {
+                                          const double* r, int cur, bool have_p, bool pending, double alpha,
+                                             double& beta, double& gamma, double& mz) {
   const MgLevel& L0 = A.lv[0];
   const FemGrid& g = L0.g;
   const uint8_t* __restrict__ pin0 = PIN ? L0.pin : nullptr;
@@ -194,9 +215,8 @@ __device__ __forceinline__ bool cg_direction(const GridTeam& gt, const GridReduc
   const double* pold = cur ? A.p1 : A.p0;
   double* __restrict__ pnew = cur ? A.p0 : A.p1;
   double* __restrict__ apo = A.Ap;
-  const double* s0 = (prec == FEM_PREC_NONE || prec == FEM_PREC_JACOBI) ? A.r : (prec == FEM_PREC_MG ? L0.t : A.z);
+  const double* s0 = (prec == FEM_PREC_NONE || prec == FEM_PREC_JACOBI) ? r : (prec == FEM_PREC_MG ? L0.t : A.z);
   const double* s1 = have_p ? pold : nullptr;
-  const double* s2 = prec == FEM_PREC_JACOBI ? L0.diag : nullptr;
   double be = beta, mzv = mz;
   auto comb = [&](const double(&v)[3]) -> double {
     double zv;
@@ -237,28 +257,34 @@ __device__ __forceinline__ bool cg_direction(const GridTeam& gt, const GridReduc
   } else {
     constexpr int nc = fem_axis_ncls(KIND, PER), S1 = 256 * KS<KIND>::NC;  // S1: from source to source in a slot
     const double* dt = smem + L0.tab_s + 2 * fem_tab_doubles(g) + fem_stencil_ncls(g);
-    fem_strip_lattice<KIND, PER, 3, 1>(
+    double* __restrict__ x = A.x;
+    fem_strip_lattice<KIND, PER, 4, 2>(
         gt, g, L0.pl, smem + L0.tab_s, smem + 128,
         [&](int i, unsigned slot) {
           fem_ring_copy(slot, s0 + i);
           if (have_p) fem_ring_copy(slot + S1, s1 + i);
           if (PIN) fem_ring_copy_mask(slot + 2 * S1, pin0, i);
+          if (have_p) fem_ring_copy(slot + 3 * S1, x + i);
         },
-        [&](int ry, int gx, int i, unsigned slot, double(&car)[1], bool& flag) {
+        [&](int ry, int gx, int i, unsigned slot, double(&car)[2], bool& flag) {
           double v[3] = {fem_ring_get(slot), have_p ? fem_ring_get(slot + S1) : 0.0, 1.0};
+          car[1] = have_p ? fem_ring_get(slot + 3 * S1) + alpha * v[1] : 0.0;
           if (prec == FEM_PREC_JACOBI)
             v[2] = dt[fem_axis_cls(KIND, PER, ry, g.ney) * nc + fem_axis_cls(KIND, PER, gx, g.nex)];
           flag = PIN && fem_ring_byte(slot + 2 * S1, i);
           car[0] = comb(v);
           return car[0];
         },
-        [&](int i, double q, const double(&car)[1], bool flag) { body(i, flag ? 0.0 : q, car[0]); },
+        [&](int i, double q, const double(&car)[2], bool flag) {
+          body(i, flag ? 0.0 : q, car[0]);
+          if (have_p) x[i] = car[1];
+        },
         [&](int it) { gr.item_sums<fem_items<KIND, PIN>(), 1>(a, slp, it); }, pre);
   }
   return gr.finish_items<fem_items<KIND, PIN>(), 1>(gt, a, slp, smem);
 }
 
-// Phase B: x += alpha p, r -= alpha Ap and the sums of r; streaming, the loads of
+// Phase B: r -= alpha Ap and the sums of r (hex8: x += alpha p too); streaming, the loads of
 // U nodes per thread in flight (the sums over 1 / D only where something reads
 // them: not under pinned multigrid)
 template <int KIND, bool PIN>
@@ -281,8 +307,10 @@ __device__ __forceinline__ bool cg_update(const GridTeam& gt, const GridReducer&
       for (int u = 0; u < U; ++u) {
         const int i = i0 + u * stride;
         if (i < end) {
-          xv[u] = x[i];
-          pv[u] = p[i];
+          if (KIND == FEM_HEX8) {
+            xv[u] = x[i];
+            pv[u] = p[i];
+          }
           rv[u] = r[i];
           av[u] = Ap[i];
           iv[u] = sums_d ? iD0[i] : 0.0;
@@ -293,7 +321,7 @@ __device__ __forceinline__ bool cg_update(const GridTeam& gt, const GridReducer&
       for (int u = 0; u < U; ++u) {
         const int i = i0 + u * stride;
         if (i < end) {
-          x[i] = xv[u] + alpha * pv[u];
+          if (KIND == FEM_HEX8) x[i] = xv[u] + alpha * pv[u];
           const double ri = rv[u] - alpha * av[u];
           r[i] = ri;
           if (put_z) A.z[i] = ri / dv[u];
@@ -370,14 +398,33 @@ __device__ __forceinline__ void cg_solve(const CgArgs& A, double* smem, unsigned
     const int prec = A.prec;
     bool have_p = false;   // after the first iteration
     int cur = 0;
+    double alpha = 0.0;
+    // the residual's update merged into the preconditioner's first phase (2D): the
+    // approximate inverse's, or the pinned V-cycle's first down-sweep if it has one.
+    // Mean-zero needs the sums of r before that phase. Separate -> merged, with x's
+    // step moved to phase A, B200: step of a channel on 90 x 33 quad9 (approximate
+    // inverse) 5735 -> 5052 us, 64^2 quad4 cavity 445 -> 436, Poisson solve on 4096^2
+    // 8204 -> 7797.
+    const bool merged = KIND != FEM_HEX8 && (prec == FEM_PREC_APPROX_INV || prec == FEM_PREC_APPROX_INV_PT ||
+                                             (prec == FEM_PREC_MG && PIN && A.nlev > 1 && A.dense_lv > 0));
+    CgResidual r0{A.r, A.Ap, prec == FEM_PREC_MG ? A.z : L0.x, 0.0, atol2, rr, false, true, false};
     const unsigned long long t_start = fem_globaltimer_early();
 #pragma unroll 1
     for (;;) {
       // z = M r; z of a final iteration is never used
-      if (have_p && prec != FEM_PREC_NONE && prec != FEM_PREC_JACOBI && !(rr > atol2 && k < A.maxiter)) break;
+      if (have_p && !merged && prec != FEM_PREC_NONE && prec != FEM_PREC_JACOBI && !(rr > atol2 && k < A.maxiter))
+        break;
       double gamma_ = 0.0;
       bool pending = false;  // MG: gamma / mz of the V-cycle are read in the next phase A
-      if (!cg_apply_prec<KIND, PIN, PER>(gt, gr, A, smem, cg_r, cg_p, cg_q, rr, r2, gamma_, mz, pending)) goto done;
+      if (!cg_apply_prec<KIND, PIN, PER>(gt, gr, A, r0, smem, cg_r, cg_p, cg_q, rr, r2, gamma_, mz, pending)) goto done;
+      if (r0.update) {
+        rr = r0.rr;
+        double* const was = const_cast<double*>(r0.r);
+        r0.r = r0.out;
+        r0.out = was;
+        r0.update = false;
+        if (r0.stop) break;
+      }
       if (!pending) {
         beta = gamma_ / gamma;
         gamma = gamma_;
@@ -385,19 +432,30 @@ __device__ __forceinline__ void cg_solve(const CgArgs& A, double* smem, unsigned
       const double rs = (prec == FEM_PREC_NONE) ? gamma : rr;
       if ((have_p && !isfinite(rs)) || !(rs > atol2 && k < A.maxiter)) break;
       if (fem_watchdog_fired(A.sync.err)) break;
-      if (!cg_direction<KIND, PIN, PER>(gt, gr, A, smem, cur, have_p, pending, beta, gamma, mz)) goto done;
+      if (!cg_direction<KIND, PIN, PER>(gt, gr, A, smem, r0.r, cur, have_p, pending, alpha, beta, gamma, mz)) goto done;
       double pap[1];
       gr.result<1>(pap, SL_PAP, smem);
       fem_watchdog_arm(A.sync.err, t_start);
-      if (!cg_update<KIND, PIN>(gt, gr, A, cur ? A.p0 : A.p1, gamma / pap[0], smem)) goto done;
+      alpha = gamma / pap[0];
       ++k;
-      double t2[2];
-      const int slrz[2] = {SL_RR, SL_RZ};
-      gr.result_slots<2>(t2, slrz, smem);
-      rr = t2[0];
-      r2 = t2[1];
+      if (merged) {
+        r0.alpha = alpha;
+        r0.more = k < A.maxiter;
+        r0.update = true;
+      } else {
+        if (!cg_update<KIND, PIN>(gt, gr, A, cur ? A.p0 : A.p1, alpha, smem)) goto done;
+        double t2[2];
+        const int slrz[2] = {SL_RR, SL_RZ};
+        gr.result_slots<2>(t2, slrz, smem);
+        rr = t2[0];
+        r2 = t2[1];
+      }
       have_p = true;
       cur ^= 1;
+    }
+    if (KIND != FEM_HEX8 && have_p) {  // the last iteration's step
+      const double* __restrict__ p = cur ? A.p1 : A.p0;
+      for (int i = gt.rank(); i < nn; i += gt.size()) A.x[i] += alpha * p[i];
     }
     // final modification of solvers/standard.py:119-123
     if (A.post) {

@@ -28,6 +28,7 @@
 #define SL_BSUM 5    // sum b (mean-zero rhs)
 #define SL_ZA 6      // r.z of the approximate inverse
 #define SL_BI 6      // BiCGSTAB: 6 rhat.r, 7 rhat.q, 8 s.s, 9 t.s, 10 t.t
+#define SL_RM 11     // r.r of a residual updated inside the preconditioner's first phase
 #define SL_LVL0 12
 #define SL_R(n) (SL_LVL0 + 6 * (n))      // 2 slots: sum R_n, sum R_n / D_n
 #define SL_T(n) (SL_LVL0 + 6 * (n) + 2)  // 1 slot : sum T_n
@@ -190,6 +191,27 @@ __device__ __forceinline__ void fem_ij(const FemGrid& g, int n, int& i, int& j, 
 struct LevelAffine {
   double alpha, beta, sum_rhD;
 };
+// The CG residual that a preconditioner reads. With `update` it is formed by the
+// preconditioner's first phase, as r - alpha Ap at every node it stages and into
+// `out` at the nodes it owns (r is read by neighbours meanwhile, hence two vectors);
+// go_on then reads r.r, and the rest of the preconditioner only runs if the solve
+// goes on. That saves the update's grid phase and one pass over r.
+struct CgResidual {
+  const double *r, *Ap;
+  double* out;
+  double alpha, limit, rr;  // limit: the loop's bound on r.r
+  bool update, more;        // more: iterations are left
+  bool stop;                // set by go_on
+  __device__ __forceinline__ const double* from() const { return r; }
+  __device__ __forceinline__ const double* now() const { return update ? out : r; }
+  __device__ __forceinline__ bool go_on(const GridReducer& gr, double* smem) {
+    double s[1];
+    gr.result<1>(s, SL_RM, smem);
+    rr = s[0];
+    stop = !(rr > limit && more);
+    return !stop;
+  }
+};
 // Per-CTA cache of each level's (alpha, beta), written by the down-sweep and
 // read back by the up-sweep of the same level (same slots, same formula).
 __device__ __forceinline__ double* fem_affine_cache() {
@@ -233,7 +255,8 @@ __device__ __forceinline__ LevelAffine fem_level_affine(const Red& red, const Cg
 // Each strip writes x_n and sums t on its coarse columns' own fine columns (2C and
 // 2C + 1). Bound by one pass over u and x_n and by the phase's barrier.
 template <int KIND, bool PIN, bool PER, class Team, class Red>
-__device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const CgArgs& A, int n, double* smem) {
+__device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const CgArgs& A, const CgResidual& r0, int n,
+                                        double* smem) {
   constexpr int NC = KS<KIND>::NC, H = KS<KIND>::H, CT = KS<KIND>::COARSE;
   fem_trace_mark(A.sync, 15);
   const MgLevel& L = A.lv[n];
@@ -248,7 +271,8 @@ __device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const Cg
   fem_level_affine_slots(n, asl);
   typename Red::template Pending<3> pend{};
   if (!pinned) pend = red.template result_begin<3>(asl);
-  const double* __restrict__ u = L.r;
+  const double* __restrict__ u = n == 0 ? r0.from() : L.r;
+  const bool upd = pinned && n == 0 && r0.update;
   const uint8_t* __restrict__ mk = L.mpin;
   double* __restrict__ xo = L.x;
   double* __restrict__ cr = C.r;
@@ -261,6 +285,8 @@ __device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const Cg
   const unsigned ring = fem_ring_lane(smem + 128);
   double acc[3] = {0.0, 0.0, 0.0};  // sum t (owned fine nodes), sum u_{n+1}, sum u_{n+1} / D_{n+1}
   const int sl[3] = {SL_T(n), SL_R(n + 1), SL_R(n + 1) + 1};
+  double arr[1] = {0.0};  // r.r of an updated residual
+  const int slm[1] = {SL_RM};
   bool first = true;
 #pragma unroll 1
   for (int it = warp * tm.ncta() + tm.cta(); first || it < P.nitem; it += nwt) {
@@ -286,19 +312,21 @@ __device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const Cg
     // full-lattice restriction does not reach below row or column 0, periodic or not)
     const int y0 = 2 * R0 - 1, y1 = act ? 2 * R1 : y0;
     double dl = 0.0, dc = 0.0, dr = 0.0, ml = 0.0, mc = 0.0, mr = 0.0;  // t of the rows below and at the coarse row
-    fem_strip<KIND, PER, pinned ? 2 * NC : NC, 2, 1>(
+    fem_strip<KIND, PER, pinned ? 3 * NC : NC, 2, 1>(
         g, tab, ring, p, y0, y1,
         [&](int, int row, unsigned slot) {
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
             fem_ring_copy(slot + c * 256, u + row + p.g[c]);
             if (pinned) fem_ring_copy_mask(slot + (NC + c) * 256, mk, row + p.g[c]);
+            if (upd) fem_ring_copy(slot + (2 * NC + c) * 256, r0.Ap + row + p.g[c]);
           }
         },
         [](int, unsigned) {},
         [&](int c, int, int ry, int i, unsigned slot, double(&car)[2], bool& flag) {
           const double d = idt[fem_axis_cls(KIND, per, ry, g.ney) * nc + kx[c]];
           double rh = fem_ring_get(slot), v;
+          if (upd) rh -= r0.alpha * fem_ring_get(slot + 2 * NC * 256);
           if (pinned) {
             flag = fem_ring_byte(slot + NC * 256, i);
             v = flag ? 0.0 : (2.0 / 3.0) * rh * d;
@@ -320,6 +348,10 @@ __device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const Cg
             tv[c] = (!in || flag[c]) ? 0.0 : car[c][0] - Lx[c];
             if (own && in && y >= 2 * R0) {
               xo[y * ux + p.x + c] = car[c][1];
+              if (upd) {
+                r0.out[y * ux + p.x + c] = car[c][0];
+                arr[0] += car[c][0] * car[c][0];
+              }
               if (!pinned) acc[0] += tv[c];
             }
           }
@@ -358,9 +390,11 @@ __device__ __forceinline__ bool mg_down(const Team& tm, const Red& red, const Cg
           }
         });
     if (!pinned && act) red.template item_sums<fem_items<KIND, PIN>(), 3>(acc, sl, it);
+    if (upd && act) red.template item_sums<fem_items<KIND, PIN>(), 1>(arr, slm, it);
     first = false;
   }
   fem_trace_mark(A.sync, 4);
+  if (upd) return red.template finish_items<fem_items<KIND, PIN>(), 1>(tm, arr, slm, smem);
   return pinned ? tm.sync() : red.template finish_items<fem_items<KIND, PIN>(), 3>(tm, acc, sl, smem);
 }
 
@@ -571,7 +605,8 @@ __device__ __forceinline__ void mg_xsums(const MgLevel& L, int i, double xi, dou
 // z = M r and the phase also accumulates the r.z pieces. Bound by one pass over
 // X_n, rhs and the result, and by the phase's barrier.
 template <int KIND, bool PIN, bool PER, class Team, class Red>
-__device__ __forceinline__ bool mg_up(const Team& tm, const Red& red, const CgArgs& A, int n, double* smem) {
+__device__ __forceinline__ bool mg_up(const Team& tm, const Red& red, const CgArgs& A, const CgResidual& r0, int n,
+                                      double* smem) {
   constexpr int R = KI<KIND>::R, NC = KS<KIND>::NC, H = KS<KIND>::H;
   fem_trace_mark(A.sync, 14);
   const MgLevel& L = A.lv[n];
@@ -586,7 +621,7 @@ __device__ __forceinline__ bool mg_up(const Team& tm, const Red& red, const CgAr
   typename Red::template Pending<2> pend{};
   if (!pinned) pend = red.template result_begin<2>(msl);
   const double* __restrict__ xi = L.x;
-  const double* __restrict__ rr = L.r;
+  const double* __restrict__ rr = n == 0 ? r0.now() : L.r;
   const double* __restrict__ xc = C.t;
   const uint8_t* __restrict__ mk = L.mpin;
   double* __restrict__ to = L.t;
@@ -728,7 +763,8 @@ __device__ __forceinline__ bool mg_up(const Team& tm, const Red& red, const CgAr
 // One warp per row, rows in blocks of 8 (a CTA's warps; a block's sums are one
 // partial column), each lane 16-byte pieces of its row, up to 8 in flight.
 template <int KIND, bool PIN>
-__device__ __forceinline__ bool mg_dense(const GridTeam& gt, const GridReducer& gr, const CgArgs& A, double* smem) {
+__device__ __forceinline__ bool mg_dense(const GridTeam& gt, const GridReducer& gr, const CgArgs& A,
+                                         const CgResidual& r0, double* smem) {
   const int d = A.dense_lv, ld = A.dense_ld, h = ld >> 1;
   const MgLevel& L = A.lv[d];
   const int n = L.g.nn, nblk = (n + 7) >> 3;
@@ -737,7 +773,7 @@ __device__ __forceinline__ bool mg_dense(const GridTeam& gt, const GridReducer& 
   if (gt.cta() < nblk) {
     double* sr = smem + 128;  // u_d (ld doubles), then the results of a block of rows
     double* sz = sr + ld;
-    fem_stage(sr, L.r, n, [](int q) { return q; });
+    fem_stage(sr, d == 0 ? r0.now() : L.r, n, [](int q) { return q; });
     for (int q = n + threadIdx.x; q < ld; q += blockDim.x) sr[q] = 0.0;
     double alpha = 0.0;
     if (!PIN && d > 0) {
@@ -804,17 +840,20 @@ __device__ __forceinline__ bool mg_dense(const GridTeam& gt, const GridReducer& 
 // 550 bytes of callee-saved registers per thread and call, 280 KB per CTA, which
 // the barriers' acquires evict from L1.
 template <int KIND, bool PIN, bool PER>
-__device__ __forceinline__ bool mg_vcycle(const GridTeam& gt, const GridReducer& gr, const CgArgs& A, double* smem,
-                                          double* cg_r, double* cg_p, double* cg_q) {
+__device__ __forceinline__ bool mg_vcycle(const GridTeam& gt, const GridReducer& gr, const CgArgs& A,
+                                          CgResidual& r0, double* smem, double* cg_r, double* cg_p, double* cg_q) {
   static_assert(KIND != FEM_HEX8, "the hex8 multigrid is k_mg3.cu");
   const int N = A.nlev;
   const bool dense = A.dense_lv < N;
   const int s = dense ? A.dense_lv : N - 1;
 #pragma unroll 1
   for (int n = 0; n < s; ++n)
-    if (!mg_down<KIND, PIN, PER>(gt, gr, A, n, smem)) return false;
+  {
+    if (!mg_down<KIND, PIN, PER>(gt, gr, A, r0, n, smem)) return false;
+    if (PIN && n == 0 && r0.update && !r0.go_on(gr, smem)) return true;
+  }
   if (dense) {
-    if (!mg_dense<KIND, PIN>(gt, gr, A, smem)) return false;
+    if (!mg_dense<KIND, PIN>(gt, gr, A, r0, smem)) return false;
   } else {
     if (blockIdx.x == 0) {
       const MgLevel& Lc = A.lv[N - 1];
@@ -843,6 +882,6 @@ __device__ __forceinline__ bool mg_vcycle(const GridTeam& gt, const GridReducer&
   }
 #pragma unroll 1
   for (int n = s - 1; n >= 0; --n)
-    if (!mg_up<KIND, PIN, PER>(gt, gr, A, n, smem)) return false;
+    if (!mg_up<KIND, PIN, PER>(gt, gr, A, r0, n, smem)) return false;
   return true;
 }

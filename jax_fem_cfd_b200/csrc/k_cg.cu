@@ -50,7 +50,8 @@ __global__ void __launch_bounds__(FEM_CG_THREADS, 1) k_vcycle(CgArgs Aparam, dou
     add(gt.rank(), nn, gt.size());
   }
   if (!gr.finish_items<fem_items<KIND, PIN>(), 2>(gt, a, slr, smem)) return;
-  if (!mg_vcycle<KIND, PIN, PER>(gt, gr, A, smem, cg_r, cg_p, cg_q)) return;
+  CgResidual r0{L0.r, nullptr, nullptr, 0.0, 0.0, 0.0, false, true, false};
+  if (!mg_vcycle<KIND, PIN, PER>(gt, gr, A, r0, smem, cg_r, cg_p, cg_q)) return;
   double sx[2];
   gr.result<2>(sx, SL_X(0), smem);
   const double mz = PIN ? 0.0 : sx[0] * L0.inv_nn;
