@@ -4,6 +4,7 @@
 #include "fem_solvers.cuh"
 #include "fem_conv.cuh"
 #include "fem_conv3.cuh"
+#include "fem_conv2.cuh"
 
 #define FEM_THREADS 512
 #define FEM_CG_THREADS 256  // k_cg / k_vcycle
@@ -12,7 +13,7 @@
 // levels' tables; at most 14 levels of 16 classes x 25 coefficients twice
 #define FEM_CG_SMEM (128 + FEM_TILE_SMEM)
 static_assert(FEM_CG_THREADS * FEM_RING_SLOTS <= FEM_TILE_SMEM, "the strips' rings fit the tile region");
-static_assert(FEM_THREADS * FEM_RING_SLOTS <= FEM_CONV_SMEM, "and the packed kernel's");
+static_assert(FEM_THREADS * FEM_RING_SLOTS <= FEM_CONV_SMEM && FEM_C2_SMEM <= FEM_CONV_SMEM, "and the packed kernel's");
 #define FEM_DYN_SMEM_MAX ((FEM_CG_SMEM + FEM_MAX_LEVELS * (2 * 400 + 2 * 16)) * 8)
 struct BiArgs {
   FemSync sync;
@@ -31,6 +32,10 @@ struct BiArgs {
   const double* cvf;
   double cv_coef;
   FemQuadTab qt;
+  // quad4, if c2U is set: the whole operator from the nodal velocities c2U (fem_conv2.cuh), by the items of c2plan
+  const double* c2U;
+  FemConv2 c2;
+  FemStripPlan c2plan;
   FemConv3 c3;  // hex8, if c3.U is set: the whole operator, applied from the nodal velocities (fem_conv3.cuh)
 };
 
@@ -55,12 +60,13 @@ struct StepArgs {
 // fem_step4 (Q1, pinned multigrid pressure, on-the-fly convection, FP64).
 struct PackMember {
   StepArgs S;  // dt and mu come from the launch's PackStep
-  BiArgs B;    // momentum solve: x = Uhat, b = rhsU; its shared matrix is built in smem
+  BiArgs B;    // momentum solve: x = Uhat, b = rhsU; its coefficients are formed per launch
   CgArgs C;    // pressure solve: b = rhsP; x is the step's output pressure
   double* U[2];
   double* P[2];
   const double* Ud;
-  double *cvf, *vcv, *rhsU, *Uhat, *gPn, *Ustar, *rhsP;
+  double hx, hy;  // element extents
+  double *vcv, *rhsU, *Uhat, *gPn, *Ustar, *rhsP;
   double *cr, *cp, *cq;
   int* stat;  // [0..1] iterations, [2..3] statuses of the last step (momentum, pressure), [4] OR of all statuses
 };
@@ -151,6 +157,9 @@ int fem_launch_conv_vjp(const FemGrid& g, const FemQuadTab& qt, int ncomp, const
 int fem_launch_transport_vjp(const FemGrid& g, const FemQuadTab& qt, const double* Un, const double* U,
                              const double* lam, const double* phin, const double* phi, double dt, double D, int supg,
                              double* gen, double* geu, double* yn, double* yu, cudaStream_t s);
+// quad4: y = (mass Me + diff Le + cc Ce(U)) x for 2 components (fem_conv2.cuh)
+int fem_launch_conv_apply2(const FemGrid& g, const FemConv2& op, const double* U, const double* x, double* y, int sms,
+                           cudaStream_t s);
 // hex8: y = (mass Me + diff Le + cc Ce(U)) x for 3 components (fem_conv3.cuh)
 int fem_launch_conv_apply3(const FemGrid& g, const FemConv3& op, const double* x, double* y, int grid, cudaStream_t s);
 

@@ -5,12 +5,13 @@
 
 // The operator apply of the solver: the element-by-element product of op on
 // load(j, c), or (OTF) on comb of the staged sources with Ce never materialised:
-// op.alpha op.A + cv_coef Ce from Gauss-point factors (2D), c3 (hex8). Identity
-// rows where A.mask is set; body(i, y, x, a) with a = aux (null: unused) at node i.
-template <int KIND, int NC, bool OTF, bool AUX, int NSRC, class Team, class Load, class Comb, class Body>
+// op.alpha op.A + cv_coef Ce from Gauss-point factors (quad9), c2 (quad4), c3 (hex8).
+// Identity rows where A.mask is set; body(i, y, x, a) with a = aux (null: unused) at
+// node i; flush(item) as fem_march_conv2's (quad4 on the fly only).
+template <int KIND, int NC, bool OTF, int SLOTS, bool AUX, int NSRC, class Team, class Load, class Comb, class Body, class Flush>
 __device__ __forceinline__ void bi_tiled_apply(const Team& tm, const BiArgs& A, const MatCombo& op, double* tsm,
                                                const Load& load, const double* const (&src)[NSRC], const Comb& comb,
-                                               const double* aux, const Body& body) {
+                                               const double* aux, const Body& body, const Flush& flush) {
   auto row = [&](int i, const double(&y)[NC], const double(&x)[NC]) {
     double v[NC], a[NC];
 #pragma unroll
@@ -23,6 +24,8 @@ __device__ __forceinline__ void bi_tiled_apply(const Team& tm, const BiArgs& A, 
   };
   if constexpr (OTF && KIND == FEM_HEX8) {
     fem_march_conv3<NSRC, AUX>(tm, A.g, tsm, src, comb, A.c3, A.mask, aux, body);
+  } else if constexpr (OTF && KIND == FEM_Q1_2D) {
+    fem_march_conv2<NSRC, AUX, SLOTS>(tm, A.g, A.c2plan, tsm, src, comb, A.c2U, A.c2, A.mask, aux, body, flush);
   } else if constexpr (OTF) {
     fem_tiled_conv<KIND, NC, NSRC>(tm, A.g, tsm, src, comb, A.cvf, A.qt, A.cv_coef, op.alpha, op.A, row);
   } else if constexpr (KIND == FEM_HEX8) {
@@ -38,12 +41,15 @@ __device__ __forceinline__ void bi_tiled_apply(const Team& tm, const BiArgs& A, 
 // The BiCGSTAB solve of k_bicgstab on the CTAs of one launch (or of one group of
 // a packed launch). op: the operator with its shared matrix (if any) already in
 // shared memory; smem: 128 doubles of reduction scratch; tsm: the tiled
-// operator's staging; s_round: the CTA's completed barriers on A.sync's counter.
-template <int KIND, int NC, bool OTF>
+// operator's staging (SLOTS: ring slots per warp of the quad4 march in it); s_round:
+// the CTA's completed barriers on A.sync's counter. Quad4 on the fly: every sum is
+// kept per work item, so the solve's bits do not depend on its CTAs.
+template <int KIND, int NC, bool OTF, int SLOTS>
 __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& op, double* smem, double* tsm,
                                                unsigned int* s_round) {
   const GridTeam gt = GridTeam::grid(&A.sync, s_round);
   const GridReducer gr{&A.sync};
+  constexpr bool ITEMS = OTF && KIND == FEM_Q1_2D;
   const int nn = A.g.nn;
   const size_t N = nn;
   int k = 0;
@@ -53,8 +59,9 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
   {
     {
       double a[2] = {0.0, 0.0};
+      const int sl[2] = {SL_BB, SL_BB + 1};
       const double* sx0[1] = {A.x};
-      bi_tiled_apply<KIND, NC, OTF, true>(gt, A, op, tsm, [&](int j, int c) { return A.x[j + c * N]; }, sx0,
+      bi_tiled_apply<KIND, NC, OTF, SLOTS, true>(gt, A, op, tsm, [&](int j, int c) { return A.x[j + c * N]; }, sx0,
                                           [](int, const double(&v)[1]) { return v[0]; }, A.b,
                                           [&](int i, const double(&Ax)[NC], const double(&)[NC],
                                               const double(&bv)[NC]) {
@@ -69,9 +76,8 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
           a[0] += bi * bi;
           a[1] += ri * ri;
         }
-      });
-      gr.reduce<2>(a, SL_BB, smem);
-      if (!gt.sync()) goto done;
+      }, [&](int it) { gr.item_sums<ITEMS, 2>(a, sl, it); });
+      if (!gr.finish_items<ITEMS, 2>(gt, a, sl, smem)) goto done;
     }
     double bb[2];
     gr.result<2>(bb, SL_BB, smem);
@@ -96,8 +102,9 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
           return r[o] + beta * (pold[o] - omega * qold[o]);
         };
         double a[1] = {0.0};
+        const int sl[1] = {SL_BI + 1};
         const double* spn[3] = {r, pold, qold};
-        bi_tiled_apply<KIND, NC, OTF, true>(gt, A, op, tsm, pn, spn,
+        bi_tiled_apply<KIND, NC, OTF, SLOTS, true>(gt, A, op, tsm, pn, spn,
                                             [&](int, const double(&v)[3]) { return v[0] + beta * (v[1] - omega * v[2]); },
                                             A.rhat, [&](int i, const double(&q)[NC], const double(&pc)[NC],
                                                         const double(&rh)[NC]) {
@@ -108,9 +115,8 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
             qnew[o] = q[c];
             a[0] += rh[c] * q[c];
           }
-        });
-        gr.reduce<1>(a, SL_BI + 1, smem);
-        if (!gt.sync()) goto done;
+        }, [&](int it) { gr.item_sums<ITEMS, 1>(a, sl, it); });
+        if (!gr.finish_items<ITEMS, 1>(gt, a, sl, smem)) goto done;
       }
       double rq[1];
       gr.result<1>(rq, SL_BI + 1, smem);
@@ -121,8 +127,9 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
       };
       {
         double a[3] = {0.0, 0.0, 0.0};
+        const int sl[3] = {SL_BI + 2, SL_BI + 3, SL_BI + 4};
         const double* ssv[2] = {r, qnew};
-        bi_tiled_apply<KIND, NC, OTF, false>(gt, A, op, tsm, sv, ssv,
+        bi_tiled_apply<KIND, NC, OTF, SLOTS, false>(gt, A, op, tsm, sv, ssv,
                                              [&](int, const double(&v)[2]) { return v[0] - alpha_ * v[1]; }, nullptr,
                                              [&](int i, const double(&tv)[NC], const double(&sc)[NC],
                                                  const double(&)[NC]) {
@@ -133,9 +140,8 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
             a[1] += tv[c] * sc[c];
             a[2] += tv[c] * tv[c];
           }
-        });
-        gr.reduce<3>(a, SL_BI + 2, smem);
-        if (!gt.sync()) goto done;
+        }, [&](int it) { gr.item_sums<ITEMS, 3>(a, sl, it); });
+        if (!gr.finish_items<ITEMS, 3>(gt, a, sl, smem)) goto done;
       }
       double st[3];
       gr.result<3>(st, SL_BI + 2, smem);
@@ -143,7 +149,8 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
       const bool exit_early = st[0] < atol2;
       {
         double a[2] = {0.0, 0.0};
-        for (int i = gt.rank(); i < nn; i += gt.size()) {
+        const int sl[2] = {SL_RR, SL_RSUM};  // SL_RSUM: rhat.r
+        auto node = [&](int i) {
           // every load before the first store, which the compiler cannot move loads across
           double s[NC], xv[NC], pv[NC], tv[NC], rh[NC];
 #pragma unroll
@@ -165,10 +172,17 @@ __device__ __forceinline__ void bicgstab_solve(const BiArgs& A, const MatCombo& 
             a[0] += rn * rn;
             a[1] += rh[c] * rn;
           }
+        };
+        if constexpr (ITEMS) {
+          fem_chunks(gt, nn, A.sync.ncols, [&](int it, int i, int end) {
+            for (; i < end; i += 32) node(i);
+            gr.item_sums<true, 2>(a, sl, it);
+          });
+        } else {
+          for (int i = gt.rank(); i < nn; i += gt.size()) node(i);
         }
-        gr.reduce<2>(a, SL_RR, smem);  // SL_RR, SL_RSUM (= rhat.r)
         fem_watchdog_arm(A.sync.err, t_start);
-        if (!gt.sync()) goto done;
+        if (!gr.finish_items<ITEMS, 2>(gt, a, sl, smem)) goto done;
       }
       double nr[2];
       gr.result<2>(nr, SL_RR, smem);

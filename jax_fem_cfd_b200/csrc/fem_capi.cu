@@ -463,7 +463,7 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   FEM_ALLOC(c->Kd, per);
   FEM_ALLOC(c->M, vn);
   FEM_ALLOC(c->Ldiag, nn);
-  FEM_ALLOC(c->dmask, vn);
+  FEM_ALLOC(c->dmask, vn + 4);  // whole words
   FEM_ALLOC(c->pmask, nn + 4);  // whole words (fem_ring_copy_mask)
   FEM_ALLOC(c->aipin, nn + 4);
   FEM_ALLOC(c->bar, 1);
@@ -1050,9 +1050,15 @@ extern "C" int fem_mg_vcycle(fem_ctx* c, const double* r, double* z, cudaStream_
   return fem_launch_vcycle(A, cg_grid_for(c), c->cr, c->cp, c->cq, z, s);
 }
 
+// Items of the quad4 momentum solve and of its sums, as many as the CG's
+static FemStripPlan bi_plan(const fem_ctx* c) {
+  return fem_strip_plan(c->g.nnx, FEM_C2_OWN, c->g.nny, cg_items(c), 1);
+}
+
 static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t* mask, const double* b, double* x,
                         double tol, double atol, int maxiter, int* iters, int* status, cudaStream_t s,
-                        const double* cvf = nullptr, double cv_coef = 0.0, const FemConv3* c3 = nullptr) {
+                        const double* cvf = nullptr, double cv_coef = 0.0, const FemConv3* c3 = nullptr,
+                        const double* c2U = nullptr, const FemConv2* c2 = nullptr) {
   if (ncomp < 1 || ncomp > c->ndim) return FEM_E_ARG;  // workspace holds ndim*nn per vector
   BiArgs A;
   memset(&A, 0, sizeof(A));
@@ -1078,10 +1084,17 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
   A.cv_coef = cv_coef;
   A.qt = c->qt;
   if (c3) A.c3 = *c3;
+  if (c2) {
+    A.c2 = *c2;
+    A.c2U = c2U;
+    A.c2plan = bi_plan(c);
+  }
   FEM_TRY(reset_sync(c, s));
-  // the hex8 march splits to single planes
-  A.sync.ncols = c3 ? (int)std::min<long long>(c->max_coop, fem_c3_units(c->g)) : ctx_grid_for(c);
-  return fem_launch_bicgstab(ncomp, A, A.sync.ncols, s);
+  // the hex8 march splits to single planes, the quad4 one to its items
+  const int grid = c3 ? (int)std::min<long long>(c->max_coop, fem_c3_units(c->g))
+                      : (c2 ? std::min(cg_items(c), c->max_coop) : ctx_grid_for(c));
+  A.sync.ncols = c2 ? cg_items(c) : grid;
+  return fem_launch_bicgstab(ncomp, A, grid, s);
 }
 
 extern "C" int fem_bicgstab_solve(fem_ctx* c, int ncomp, double alpha, const double* Ash, double beta,
@@ -1108,15 +1121,21 @@ extern "C" int fem_step4(fem_ctx* c, const double* Un, const double* Pn, double 
   c->nev = 0;
   stage_mark(c, s);
   // 1. Ce(U_n), beta = 1/2 (solvers/standard.py:152). On the fly: Ce is never
-  // built; its Gauss-point factors are, and (mu Le + rho Ce) U_n of the momentum
-  // rhs is applied here.
+  // built (quad9: its Gauss-point factors are), and (mu Le + rho Ce) U_n of the
+  // momentum rhs is applied here.
   const bool otf = c->conv_otf && (c->cvf || g.kind == FEM_HEX8);
   const double hx = c->lx / g.nex, hy = c->ly / g.ney, hz = g.kind == FEM_HEX8 ? c->lz / g.nez : 0.0;  // of a hex8 box
   if (otf && g.kind == FEM_HEX8) {
     FEM_TRY(fem_launch_conv_apply3(g, fem_conv3_coef(Un, hx, hy, hz, rho, 0.5, 0.0, mu), Un, c->vcv, c->sms, s));
   } else if (otf) {
-    FEM_TRY(fem_launch_conv_factors(g, c->qt, Un, 0.5, c->cvf, s));
-    FEM_TRY(fem_launch_conv_apply(2, g, c->qt, c->cvf, rho, mu, c->Le, Un, c->vcv, c->sms, s));
+    // factors: the quad9 operator's, and the mixed-precision solve's
+    const bool q1 = g.kind == FEM_Q1_2D;
+    if (!q1 || c->precision == FEM_PRECISION_MIXED)
+      FEM_TRY(fem_launch_conv_factors(g, c->qt, Un, 0.5, c->cvf, s));
+    if (q1)
+      FEM_TRY(fem_launch_conv_apply2(g, fem_conv2_coef(hx, hy, rho, 0.5, 0.0, mu), Un, Un, c->vcv, c->sms, s));
+    else
+      FEM_TRY(fem_launch_conv_apply(2, g, c->qt, c->cvf, rho, mu, c->Le, Un, c->vcv, c->sms, s));
   } else {
     FEM_TRY(fem_launch_convection(g, quad_of(c), Un, 0.5, 0, c->Ce, s));
   }
@@ -1144,7 +1163,9 @@ extern "C" int fem_step4(fem_ctx* c, const double* Un, const double* Pn, double 
   S.pinned = c->set_zeroP;
   FEM_TRY(fem_launch_mom_rhs(S, Un, Pn, Ud, F, c->rhsU, c->Uhat, c->gPn, s));
   // 3. BiCGSTAB on (rho/dt) Me + theta (rho Ce + mu Le), identity rows on gamma_d (:20-28, :41)
-  FEM_TRY(fem_launch_lincomb(nen * nen, rho / dt, c->Me, theta * mu, c->Le, c->Kd, s));
+  // its shared matrix, for the forms that are not marched from U_n
+  if (!otf || g.kind == FEM_Q2_2D || (g.kind == FEM_Q1_2D && c->precision == FEM_PRECISION_MIXED))
+    FEM_TRY(fem_launch_lincomb(nen * nen, rho / dt, c->Me, theta * mu, c->Le, c->Kd, s));
   stage_mark(c, s);
   if (otf && c->precision == FEM_PRECISION_MIXED && g.kind != FEM_HEX8) {
     // FP64 refinement around FP32 BiCGSTAB iterations (k_mixmom.cu)
@@ -1156,6 +1177,10 @@ extern "C" int fem_step4(fem_ctx* c, const double* Un, const double* Pn, double 
     const FemConv3 op = fem_conv3_coef(Un, hx, hy, hz, theta * rho, 0.5, rho / dt, theta * mu);
     FEM_TRY(run_bicgstab(c, nd, MatCombo{}, S.dmask, c->rhsU, c->Uhat, tol, 0.0, 0, iters, status, s, nullptr, 0.0,
                          &op));
+  } else if (otf && g.kind == FEM_Q1_2D) {
+    const FemConv2 op = fem_conv2_coef(hx, hy, theta * rho, 0.5, rho / dt, theta * mu);
+    FEM_TRY(run_bicgstab(c, nd, MatCombo{}, S.dmask, c->rhsU, c->Uhat, tol, 0.0, 0, iters, status, s, nullptr, 0.0,
+                         nullptr, Un, &op));
   } else if (otf) {
     const MatCombo op{c->Kd, 1.0, nullptr, 0.0, 0, nullptr, 0.0};
     FEM_TRY(run_bicgstab(c, nd, op, S.dmask, c->rhsU, c->Uhat, tol, 0.0, 0, iters, status, s, c->cvf, theta * rho));
@@ -1650,9 +1675,8 @@ extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, d
     B.maxiter = 10 * 2 * c->g.nn;  // utils/jax_iterative_solvers.py:181-183
     B.iters = st;
     B.status = st + 2;
-    B.cvf = c->cvf;
-    B.cv_coef = theta * rho;
-    B.qt = c->qt;
+    B.c2plan = bi_plan(c);
+    B.sync.ncols = cg_items(c);
     // the pressure solve of run_cg (x is the step's output pressure)
     CgArgs& C = M.C;
     fill_cg_args(c, C);
@@ -1674,7 +1698,8 @@ extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, d
     M.P[0] = P0[m];
     M.P[1] = P1[m];
     M.Ud = c->has_dmask ? Ud[m] : nullptr;
-    M.cvf = c->cvf;
+    M.hx = c->lx / c->g.nex;
+    M.hy = c->ly / c->g.ney;
     M.vcv = c->vcv;
     M.rhsU = c->rhsU;
     M.Uhat = c->Uhat;

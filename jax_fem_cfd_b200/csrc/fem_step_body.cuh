@@ -207,6 +207,23 @@ __device__ __forceinline__ void step_conv_factors(const FemGrid& g, const FemQua
   }
 }
 
+// quad4: y = (mass Me + diff Le + cc Ce(U)) x over the whole lattice by the items of
+// plan (sm: SLOTS ring slots per warp)
+template <int SLOTS, class Team>
+__device__ __forceinline__ void step_conv_apply2(const Team& tm, const FemGrid& g, const FemStripPlan& plan,
+                                                 const FemConv2& op, const double* __restrict__ U,
+                                                 const double* __restrict__ x, double* __restrict__ y, double* sm) {
+  const size_t nn = g.nn;
+  const double* src[1] = {x};
+  fem_march_conv2<1, 0, SLOTS>(tm, g, plan, sm, src, [](int, const double(&v)[1]) { return v[0]; }, U, op, nullptr,
+                               nullptr,
+                               [&](int i, const double(&v)[2], const double(&)[2], const double(&)[2]) {
+#pragma unroll
+                                 for (int c = 0; c < 2; ++c) y[i + c * nn] = v[c];
+                               },
+                               [](int) {});
+}
+
 // y = alpha Ash x + cc Ce x over the whole lattice, the tiles dealt over the CTAs
 // (sA: Ash in shared memory or null; sm: FEM_CONV_SMEM doubles).
 template <int KIND, int NC>

@@ -3,7 +3,7 @@
 
 
 __host__ __device__ constexpr int bi_threads(int kind, bool otf) {
-  return otf && kind == FEM_HEX8 ? FEM_C3_THREADS : FEM_THREADS;
+  return otf && kind == FEM_HEX8 ? FEM_C3_THREADS : (otf && kind == FEM_Q1_2D ? FEM_C2_THREADS : FEM_THREADS);
 }
 
 template <int KIND, int NC, bool OTF>
@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(bi_threads(KIND, OTF), 1) k_bicgstab(const __g
   if (threadIdx.x == 0) s_round = 0u;
   fem_trace_init(A.sync);
   __syncthreads();
-  bicgstab_solve<KIND, NC, OTF>(A, op, smem, tsm, &s_round);
+  bicgstab_solve<KIND, NC, OTF, FEM_C2_SLOTS>(A, op, smem, tsm, &s_round);
 }
 
 static const void* bi_fn(int kind, int ncomp, bool otf) {
@@ -46,7 +46,7 @@ static int bi_smem_doubles(int kind, int ncomp, bool otf) {
 int fem_launch_bicgstab(int ncomp, const BiArgs& A, int grid, cudaStream_t s) {
   BiArgs a = A;
   void* args[] = {&a};
-  const bool otf = A.g.kind == FEM_HEX8 ? A.c3.U != nullptr : A.cvf != nullptr;
+  const bool otf = A.c3.U || A.c2U || A.cvf;
   if (otf && ncomp != (A.g.kind == FEM_HEX8 ? 3 : 2)) return FEM_E_ARG;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);

@@ -956,6 +956,24 @@ int fem_launch_conv_apply(int ncomp, const FemGrid& g, const FemQuadTab& qt, con
   return fem_after_launch("k_conv_apply");
 }
 
+// quad4: y = (mass Me + diff Le + cc Ce(U)) x for 2 components
+__global__ void __launch_bounds__(FEM_C2_THREADS, 1)
+    k_conv_apply2(FemGrid g, const __grid_constant__ FemStripPlan plan, const __grid_constant__ FemConv2 op,
+                  const double* __restrict__ U, const double* __restrict__ x, double* __restrict__ y) {
+  extern __shared__ __align__(128) double sm2[];
+  step_conv_apply2<FEM_C2_SLOTS>(FemCtaTeam{}, g, plan, op, U, x, y, sm2);
+}
+
+int fem_launch_conv_apply2(const FemGrid& g, const FemConv2& op, const double* U, const double* x, double* y, int sms,
+                           cudaStream_t s) {
+  if (g.kind != FEM_Q1_2D || sms < 1) return FEM_E_ARG;
+  const int dyn = FEM_C2_SMEM * (int)sizeof(double);
+  cudaFuncSetAttribute(k_conv_apply2, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+  const FemStripPlan plan = fem_strip_plan(g.nnx, FEM_C2_OWN, g.nny, sms * (FEM_C2_THREADS / 32), 1);
+  k_conv_apply2<<<std::min(sms, plan.nitem), FEM_C2_THREADS, dyn, s>>>(g, plan, op, U, x, y);
+  return fem_after_launch("k_conv_apply2");
+}
+
 // hex8: y = (mass Me + diff Le + cc Ce(U)) x for 3 components
 __global__ void __launch_bounds__(FEM_C3_THREADS, 1)
     k_conv_apply3(FemGrid g, const __grid_constant__ FemConv3 op, const double* __restrict__ x, double* __restrict__ y) {

@@ -11,7 +11,7 @@
 //
 // The step (solvers/standard.py:148-165, theta = 1/2, rho = 1, Ce(U_n) with
 // beta = 1/2 applied on the fly, pinned pressure with the multigrid V-cycle):
-//   1. Gauss-point factors of Ce(U_n); (mu Le + Ce) U_n
+//   1. (mu Le + Ce(U_n)) U_n
 //   2. momentum rhs and x0, G P_n
 //   3. BiCGSTAB on (1/dt) Me + theta (Ce + mu Le), identity rows on gamma_d
 //   4. U* = U_hat + dt G P_n / M
@@ -22,7 +22,7 @@
 #include "fem_bicgstab_body.cuh"
 #include "fem_step_body.cuh"
 
-// dynamic smem (doubles): [0,128) reductions | tiles of the convection apply,
+// dynamic smem (doubles): [0,128) reductions | rings of the convection apply,
 // the BiCGSTAB operator and the CG phases | CG stencil tables (quad4)
 #define FEM_PACK_SMEM (128 + FEM_CONV_SMEM + FEM_MAX_LEVELS * (2 * 81 + 2 * 9))
 static_assert(FEM_CONV_SMEM >= FEM_TILE_SMEM, "the tile region holds the CG tiles too");
@@ -34,9 +34,7 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
   __shared__ __align__(16) CgArgs sC;
   __shared__ __align__(16) BiArgs sB;
   __shared__ __align__(16) StepArgs sS;
-  __shared__ double sKd[81], sLe[81];
   __shared__ unsigned int s_round;
-  constexpr int NEN = KI<KIND>::NEN;
   const int mi = P.idx[blockIdx.y];  // the member this group runs
   const PackStep ps = P.m[mi];
   if (ps.steps <= 0) return;  // (not launched by fem_pack_step; a group with nothing to do leaves)
@@ -46,13 +44,8 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
   fem_stage_args(M.S, &sS);
   fem_tables_to_smem(sC, smem, 128 + FEM_CONV_SMEM);
   const double theta = 0.5, rho = 1.0, dt = ps.dt, mu = ps.mu;
-  // the momentum operator's shared matrix (the solo step's k_lincomb expression)
-  const double ka = rho / dt, kb = theta * mu;
-  for (int t = threadIdx.x; t < NEN * NEN; t += blockDim.x) {
-    sKd[t] = ka * sS.Me[t] + kb * sS.Le[t];
-    sLe[t] = sS.Le[t];
-  }
   if (threadIdx.x == 0) {
+    sB.c2 = fem_conv2_coef(M.hx, M.hy, theta * rho, 0.5, rho / dt, theta * mu);  // as the solo step's
     s_round = 0u;
     sS.dt = dt;
     sS.mu = mu;
@@ -60,7 +53,7 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
     sS.theta = theta;
   }
   __syncthreads();
-  const MatCombo op{sKd, 1.0, nullptr, 0.0, 0, nullptr, 0.0};
+  const FemConv2 rhs_op = fem_conv2_coef(M.hx, M.hy, rho, 0.5, 0.0, mu);
   const GridTeam gt = GridTeam::grid(&sC.sync, &s_round);
   const size_t nn = sS.g.nn;
   int* stat = M.stat;
@@ -72,16 +65,15 @@ __global__ void __launch_bounds__(FEM_THREADS, 1) k_step_pack(const PackMember* 
     double* Pn = M.P[cur];
     double* Uo = M.U[cur ^ 1];
     double* Po = M.P[cur ^ 1];
-    // 1. Ce(U_n) factors (beta = 1/2), then (mu Le + rho Ce) U_n
-    step_conv_factors<KIND>(sS.g, sB.qt, Un, 0.5, M.cvf);
-    if (!gt.sync()) return;
-    step_conv_apply<KIND, 2>(sS.g, sB.qt, M.cvf, rho, mu, sLe, Un, M.vcv, smem + 128);
+    // 1. (mu Le + rho Ce(U_n)) U_n, beta = 1/2
+    step_conv_apply2<FEM_RING_SLOTS>(gt, sS.g, sB.c2plan, rhs_op, Un, Un, M.vcv, smem + 128);
+    if (threadIdx.x == 0) sB.c2U = Un;
     if (!gt.sync()) return;
     // 2. momentum rhs, x0 and G P_n
     step_mom_rhs<KIND>(sS, Un, Pn, M.Ud, nullptr, M.rhsU, M.Uhat, M.gPn);
     if (!gt.sync()) return;
     // 3. momentum BiCGSTAB (ends on a barrier)
-    bicgstab_solve<KIND, 2, true>(sB, op, smem, smem + 128, &s_round);
+    bicgstab_solve<KIND, 2, true, FEM_RING_SLOTS>(sB, MatCombo{}, smem, smem + 128, &s_round);
     // 4. U*
     step_ustar((int)(2 * nn), dt / rho, M.Uhat, M.gPn, sS.M, M.Ustar);
     if (!gt.sync()) return;
