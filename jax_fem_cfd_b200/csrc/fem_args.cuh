@@ -218,7 +218,8 @@ int fem_coop_occupancy_cg(int* occ);
 int fem_coop_occupancy_bi(int* occ);
 int fem_launch_cg(const CgArgs& A, int grid, double* cr, double* cp, double* cq, cudaStream_t s);
 int fem_launch_vcycle(const CgArgs& A, int grid, double* cr, double* cp, double* cq, double* z, cudaStream_t s);
-int fem_launch_bicgstab(int ncomp, const BiArgs& A, int grid, cudaStream_t s);
+// threads: of a block, at most the kernel's own (at least 8 warps)
+int fem_launch_bicgstab(int ncomp, const BiArgs& A, int grid, int threads, cudaStream_t s);
 // packed step (k_pack.cu): k members of `ctas` CTAs each, one cooperative launch
 int fem_launch_step_pack(int kind, int periodic, const PackMember* members, const PackParams& P, int k, int ctas,
                          cudaStream_t s);

@@ -1091,10 +1091,22 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
   }
   FEM_TRY(reset_sync(c, s));
   // the hex8 march splits to single planes, the quad4 one to its items
-  const int grid = c3 ? (int)std::min<long long>(c->max_coop, fem_c3_units(c->g))
-                      : (c2 ? std::min(cg_items(c), c->max_coop) : ctx_grid_for(c));
+  int grid = ctx_grid_for(c), threads = FEM_THREADS;
+  if (c3) {
+    grid = (int)std::min<long long>(c->max_coop, fem_c3_units(c->g));
+  } else if (c2) {
+    grid = std::min(cg_items(c), c->max_coop);
+  } else if (!cvf && c->g.kind != FEM_HEX8) {
+    // explicit element matrices, tiles of 32 columns and a row per warp: where tiles of
+    // 16 rows leave CTAs idle, 8 rows and a tile per CTA
+    const long long ntx = (c->g.nnx + 31) / 32;
+    if (ntx * ((c->g.nny + 15) / 16) < c->max_coop) {
+      threads = 256;
+      grid = (int)std::min<long long>(c->max_coop, ntx * ((c->g.nny + 7) / 8));
+    }
+  }
   A.sync.ncols = c2 ? cg_items(c) : grid;
-  return fem_launch_bicgstab(ncomp, A, grid, s);
+  return fem_launch_bicgstab(ncomp, A, grid, threads, s);
 }
 
 extern "C" int fem_bicgstab_solve(fem_ctx* c, int ncomp, double alpha, const double* Ash, double beta,

@@ -43,14 +43,14 @@ static int bi_smem_doubles(int kind, int ncomp, bool otf) {
   return 3 * 1836;
 }
 
-int fem_launch_bicgstab(int ncomp, const BiArgs& A, int grid, cudaStream_t s) {
+int fem_launch_bicgstab(int ncomp, const BiArgs& A, int grid, int threads, cudaStream_t s) {
   BiArgs a = A;
   void* args[] = {&a};
   const bool otf = A.c3.U || A.c2U || A.cvf;
   if (otf && ncomp != (A.g.kind == FEM_HEX8 ? 3 : 2)) return FEM_E_ARG;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(bi_threads(A.g.kind, otf));
+  cfg.blockDim = dim3(std::min(threads, bi_threads(A.g.kind, otf)));
   cfg.stream = s;
   cfg.dynamicSmemBytes = (size_t)bi_smem_doubles(A.g.kind, ncomp, otf) * sizeof(double);
   cudaLaunchAttribute at[1];
