@@ -119,21 +119,22 @@ class ClockSampler:
 def cg_algorithmic_bytes(level_nn, iters, block_from):
     """Algorithmic DRAM bytes of one k_cg launch (MG-PCG, mean-zero). Per phase:
     the nn-length vectors it must read and write once (FP64), stencil re-reads
-    excluded. Init: b, x0 -> r (+centred rhs copy): 5 nn. Per iteration: p/Ap
-    phase reads z, p_old, writes p_new, Ap (4 nn); x/r update reads x, p, r, Ap,
-    diag and writes x, r (7 nn). Per V-cycle level n: pre-smooth+residual
-    reads r, diag, writes x, t (4 nn_n); restriction reads t and diag_{n+1},
-    writes r_{n+1} (nn_n + 2 nn_{n+1}); prolongation reads x_{n+1}, x, writes
-    t (2 nn_n + nn_{n+1}); post-smooth reads t, r, diag, writes x (4 nn_n).
-    The V-cycle of the final iteration is skipped (its z is never used)."""
+    excluded. Init: b, x0 -> r: 3 nn. Per iteration: the direction phase reads z,
+    p_old, x and writes p, Ap, x (6 nn); the residual update reads r, Ap, diag and
+    writes r (4 nn). Per V-cycle level n above the dense one: the down-sweep reads
+    r, writes x and r_{n+1} (2 nn_n + nn_{n+1}); the up-sweep reads x, r, x_{n+1},
+    writes t (3 nn_n + nn_{n+1}). The first level of at most 1,700 nodes is a dense
+    product: its matrix, r and t. The V-cycle of the final iteration is skipped (its
+    z is never used); x takes its last step at the end (3 nn)."""
     w = 8
-    L = len(level_nn)
     vcyc = 0
-    for n in range(L - 1):
-        vcyc += 11 * level_nn[n] + 3 * level_nn[n + 1]
-    vcyc += 3 * level_nn[-1]
+    for n, m in enumerate(level_nn):
+        if m <= 1700:
+            vcyc += m * m + 2 * m
+            break
+        vcyc += 5 * m + (2 * level_nn[n + 1] if n + 1 < len(level_nn) else 0)
     nn = level_nn[0]
-    total = 5 * nn + vcyc + iters * (11 * nn) + max(iters - 1, 0) * vcyc + 2 * nn
+    total = 3 * nn + vcyc + iters * (10 * nn) + max(iters - 1, 0) * vcyc + 3 * nn
     return total * w
 
 
@@ -682,7 +683,7 @@ def mg3_vcycle(nx=256, reps=20, warmup=3):
 def cg_trace(size=256):
     """Phase timeline of one pressure solve of the Taylor-Green step (size^2
     Q2, after 5 warm-up steps): CTA 0 of the persistent solvers stamps
-    %globaltimer at every grid (tag 31) or team (tag 30) barrier and at the
+    %globaltimer at every grid barrier (tag 31) and at the
     multigrid phase marks (fem_ctx_set_trace), and the gaps between
     consecutive marks are summed by (from, to) tag pair. The trace costs a few
     percent of the solve; the totals are for reading the phase structure, not
