@@ -228,6 +228,14 @@ static int dense_level(const fem_ctx* c, const double** C, int* ld) {
 // ctx_grid_for CTAs of 16 warps, at most one round of the whole device.
 static int cg_items(const fem_ctx* c) { return std::min(ctx_grid_for(c) * 16, c->sms * (FEM_CG_THREADS / 32)); }
 
+// Columns of a slot that any solve of the context may use: a column per CTA, or per
+// item. A plan never has fewer items than strips, so a wide lattice on a small CTA
+// cap has more of them than cg_items; the quad4 momentum strips are the narrowest.
+static int max_columns(const fem_ctx* c) {
+  const int strips = c->g.kind == FEM_Q1_2D ? (c->g.nnx + FEM_C2_OWN - 1) / FEM_C2_OWN : 0;
+  return std::max({c->coop_capacity, c->sms * (FEM_CG_THREADS / 32), strips});
+}
+
 // CTAs of a CG solve: one warp of work per CTA while there are items (a warp
 // alone on its SM runs fastest: 64^2 quad4 cavity step on 9 CTAs 541 us, on 145
 // 373 us), and enough for the dense level's rows.
@@ -443,7 +451,7 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   c->max_coop = c->sms * occ;
   const char* ev = getenv("FEM_MAX_CTAS");
   if (ev && atoi(ev) > 0) c->max_coop = std::min(c->max_coop, atoi(ev));
-  c->coop_capacity = c->max_coop;  // partials are sized for this many CTAs
+  c->coop_capacity = c->max_coop;
   const FemGrid& g = c->g;
   c->ndim = (g.kind == FEM_HEX8) ? 3 : 2;
   c->nq = g.nen;
@@ -468,7 +476,7 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   FEM_ALLOC(c->aipin, nn + 4);
   FEM_ALLOC(c->bar, 1);
   FEM_ALLOC(c->err, 1);
-  FEM_ALLOC(c->partials, (size_t)FEM_NSLOTS * std::max(c->max_coop, c->sms * (FEM_CG_THREADS / 32)));
+  FEM_ALLOC(c->partials, (size_t)FEM_NSLOTS * max_columns(c));
   FEM_ALLOC(c->flags, 16);
   for (double** p : {&c->pr, &c->pz, &c->pp0, &c->pp1, &c->pAp, &c->rhsP}) FEM_ALLOC(*p, nn);
   for (double** p : {&c->br, &c->brh, &c->bp0, &c->bp1, &c->bq0, &c->bq1, &c->bt, &c->rhsU, &c->Uhat, &c->gPn,
@@ -928,7 +936,7 @@ static void set_cg_plan(const fem_ctx* c, CgArgs& A) {
   if (c->g.kind == FEM_HEX8) return;
   const bool by_items = cg_by_items(c);
   const int grid = cg_grid_for(c), items = by_items ? cg_items(c) : grid * (FEM_CG_THREADS / 32);
-  A.sync.ncols = by_items ? items : grid;
+  int cols = items;  // of a solve by items: as many as the largest plan has items
   for (int l = 0; l < A.nlev; ++l) {
     MgLevel& M = A.lv[l];
     const bool q2 = M.g.kind == FEM_Q2_2D;
@@ -937,11 +945,12 @@ static void set_cg_plan(const fem_ctx* c, CgArgs& A) {
     if (l + 1 < A.nlev)
       M.pd = fem_strip_plan(A.lv[l + 1].g.nnx, q2 ? KS<FEM_Q2_2D>::COARSE : KS<FEM_Q1_2D>::COARSE,
                             A.lv[l + 1].g.nny, items, 1);
+    cols = std::max({cols, M.pl.nitem, M.pd.nitem});
   }
   A.dense_lv = dense_level(c, &A.dense_C, &A.dense_ld);
   // mg_dense leaves a sum per block of 8 rows
-  if (by_items && A.dense_lv < A.nlev)
-    A.sync.ncols = std::max(items, (A.lv[A.dense_lv].g.nn + 7) / 8);
+  if (A.dense_lv < A.nlev) cols = std::max(cols, (A.lv[A.dense_lv].g.nn + 7) / 8);
+  A.sync.ncols = by_items ? cols : grid;
 }
 
 static int reset_sync(fem_ctx* c, cudaStream_t s) {
@@ -1050,10 +1059,11 @@ extern "C" int fem_mg_vcycle(fem_ctx* c, const double* r, double* z, cudaStream_
   return fem_launch_vcycle(A, cg_grid_for(c), c->cr, c->cp, c->cq, z, s);
 }
 
-// Items of the quad4 momentum solve and of its sums, as many as the CG's
+// Items of the quad4 momentum solve, as many as the CG's, and the columns of its sums
 static FemStripPlan bi_plan(const fem_ctx* c) {
   return fem_strip_plan(c->g.nnx, FEM_C2_OWN, c->g.nny, cg_items(c), 1);
 }
+static int bi_columns(const fem_ctx* c, const FemStripPlan& plan) { return std::max(cg_items(c), plan.nitem); }
 
 static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t* mask, const double* b, double* x,
                         double tol, double atol, int maxiter, int* iters, int* status, cudaStream_t s,
@@ -1105,7 +1115,7 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
       grid = (int)std::min<long long>(c->max_coop, ntx * ((c->g.nny + 7) / 8));
     }
   }
-  A.sync.ncols = c2 ? cg_items(c) : grid;
+  A.sync.ncols = c2 ? bi_columns(c, A.c2plan) : grid;
   return fem_launch_bicgstab(ncomp, A, grid, threads, s);
 }
 
@@ -1688,7 +1698,7 @@ extern "C" int fem_pack_create(fem_ctx* const* ctxs, int k, double* const* U0, d
     B.iters = st;
     B.status = st + 2;
     B.c2plan = bi_plan(c);
-    B.sync.ncols = cg_items(c);
+    B.sync.ncols = bi_columns(c, B.c2plan);
     // the pressure solve of run_cg (x is the step's output pressure)
     CgArgs& C = M.C;
     fill_cg_args(c, C);
