@@ -110,7 +110,9 @@ int fem_ctx_element_data(const fem_ctx* ctx, double* wq, double* N, double* Nder
 /* Boundary sets. dmask: uint8 (ndim*nn), 1 on gamma_d entries
  * (setup/simulation.py:169-173). pmask: uint8 (nn), 1 on gamma_p nodes (outlet
  * nodes, or node 0 when there is no outlet: setup/simulation.py:178-181).
- * set_zeroP selects pinned (1) or mean-zero (0) pressure (StandardSolverConfig). */
+ * set_zeroP selects pinned (1) or mean-zero (0) pressure (StandardSolverConfig).
+ * The sets are rewritten in place: a captured step or a pack made before keeps
+ * its pressure mode and reads the new ones. */
 int fem_ctx_set_bc(fem_ctx* ctx, const uint8_t* dmask, const uint8_t* pmask, int set_zeroP, cudaStream_t stream);
 
 /* Multigrid hierarchy (core/multigrid.py:9-88): nlev levels obtained by halving
@@ -123,7 +125,8 @@ int fem_ctx_set_bc(fem_ctx* ctx, const uint8_t* dmask, const uint8_t* pmask, int
  * and R = P^T, a degree-3 Chebyshev smoother on D^-1 A with its interval from
  * a power-iteration estimate of lambda_max, and the coarsest level (at most
  * 4096 nodes) solved exactly by its inverse, formed on the device here;
- * coarse_tol is then unused. Pinned pressure only. */
+ * coarse_tol is then unused. Pinned pressure only. A call replaces the
+ * hierarchy: captured steps and packs made before it must not run again. */
 int fem_ctx_setup_multigrid(fem_ctx* ctx, int nlev, const uint8_t* level_pmasks, double coarse_tol,
                             cudaStream_t stream);
 

@@ -204,13 +204,17 @@ struct FemDenseLevel {
   const double *tab, *tab_off, *invD;  // invD: 1 / diag, 0 on gamma_p (pinned)
   const uint8_t* pin;                  // pinned mode, else null
 };
+inline int fem_dense_ld(int n) { return (n + 3) & ~3; }  // rows start on 32 bytes
 struct FemDense;  // shared by the contexts whose coarse levels are the same
 // The matrices of lv[0..nlev) (finest first; the whole hierarchy from some level
-// down), from the registry or built on stream s; *out owns a reference. FEM_OK
-// with *out null where no level qualifies.
+// down, pinned: from level 1 at most), from the registry or built on stream s;
+// *out owns a reference. FEM_OK with *out null where no level qualifies.
 int fem_dense_acquire(FemDense** out, const FemDenseLevel* lv, int nlev, int pinned, double lx, double ly, int device,
                       int sms, cudaStream_t s);
 void fem_dense_release(FemDense* d);
+// The pinned operator of level lv[0] into C (n x ld) from the matrix Cc of lv[1],
+// on stream s without waiting for it: lv[0].invD carries the current pins.
+int fem_dense_finest(const FemDenseLevel* lv, const double* Cc, int ldc, double* C, int ld, int sms, cudaStream_t s);
 // matrix and row pitch of the level with `from_end` levels below it, null if none
 const double* fem_dense_matrix(const FemDense* d, int from_end, int* ld);
 

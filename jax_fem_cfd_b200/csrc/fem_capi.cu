@@ -124,7 +124,12 @@ struct fem_ctx {
   int nlev = 0;
   double coarse_tol = 1e-8;
   CtxLevel lv[FEM_MAX_LEVELS];
-  FemDense* dense = nullptr;      // dense operators of the coarse levels (2D), shared between contexts
+  // dense operators of the coarse levels (2D) by pressure mode (mean-zero, pinned), shared
+  // between contexts; of level 0 in pinned mode, rewritten in place by fem_ctx_set_bc. Both
+  // live as long as the hierarchy: captured graphs and packs point at them.
+  FemDense* dense[2] = {};
+  bool dense_made[2] = {};
+  double* dense0 = nullptr;
   const uint8_t* pin0 = nullptr;  // the gamma_p mask that level 0's winvD was made from
   double *cr = nullptr, *cp = nullptr, *cq = nullptr;  // coarse CG scratch
   // barrier / reduction state
@@ -198,7 +203,7 @@ static int dalloc(T** p, size_t n) {
 // Whether the pressure solve may use the dense coarse operators: always on a
 // mean-zero hierarchy (the same linear map), on a pinned one when the coarsest
 // CG is asked for at least six digits, so that the exact inverse stands for it.
-static bool dense_usable(const fem_ctx* c) { return c->dense && (!c->set_zeroP || c->coarse_tol <= 1e-6); }
+static bool dense_usable(const fem_ctx* c) { return !c->set_zeroP || c->coarse_tol <= 1e-6; }
 
 // CTAs of the persistent BiCGSTAB and of a packed member: ~1 node per thread, capped
 // by co-residency.
@@ -218,7 +223,11 @@ static int dense_level(const fem_ctx* c, const double** C, int* ld) {
   if (dense_usable(c))
     for (int l = 0; l < c->nlev; ++l) {
       const long long n = c->lv[l].g.nn;
-      *C = fem_dense_matrix(c->dense, c->nlev - 1 - l, ld);
+      *C = fem_dense_matrix(c->dense[c->set_zeroP], c->nlev - 1 - l, ld);
+      if (l == 0 && c->set_zeroP) {
+        *C = c->dense0;
+        *ld = fem_dense_ld((int)n);
+      }
       if (*C && (n * n <= dense_ctas(c) * FEM_DENSE_ENTRIES || (c->set_zeroP && l == c->nlev - 1))) return l;
     }
   return c->nlev;
@@ -326,6 +335,16 @@ static int element_setup(const FemGrid& g, double dx, double dy, double dz, doub
 
 // ------------------------------------------------------------ context ----
 
+static void dense_drop(fem_ctx* c) {
+  for (int m = 0; m < 2; ++m) {
+    fem_dense_release(c->dense[m]);
+    c->dense[m] = nullptr;
+    c->dense_made[m] = false;
+  }
+  if (c->dense0) cudaFree(c->dense0);
+  c->dense0 = nullptr;
+}
+
 extern "C" void fem_ctx_destroy(fem_ctx* c) {
   if (!c) return;
   int prev = 0;
@@ -341,7 +360,7 @@ extern "C" void fem_ctx_destroy(fem_ctx* c) {
   mg3_destroy(c->mg3);
   mg3_destroy(c->mg2);
   mixmom_destroy(c->mixmom);
-  fem_dense_release(c->dense);
+  dense_drop(c);
   void* ptrs[] = {c->coords, c->wq, c->N, c->dN, c->Me, c->Le, c->Leoff, c->Ge, c->M, c->Ldiag, c->Kd,
                   c->dmask, c->pmask, c->aipin, c->cr, c->cp, c->cq, c->bar, c->err, c->partials, c->pr,
                   c->pz, c->pp0, c->pp1, c->pAp, c->br, c->brh, c->bp0, c->bp1, c->bq0, c->bq1, c->bt,
@@ -600,24 +619,44 @@ extern "C" int fem_ctx_element_data(const fem_ctx* c, double* wq, double* N, dou
   return FEM_OK;
 }
 
-// The dense coarse operators of the current hierarchy and pressure mode (2D).
-// A context without them (no level small enough, no memory for them) solves its
-// coarsest level in CTA 0.
-static int dense_refresh(fem_ctx* c, cudaStream_t s) {
-  if (c->g.kind == FEM_HEX8 || c->nlev < 2) return FEM_OK;
+static FemDenseLevel dense_level_of(const fem_ctx* c, int l) {
+  const CtxLevel& L = c->lv[l];
+  return FemDenseLevel{L.g, lattice_of(L.g), L.tab, L.tab_off, c->set_zeroP ? L.winvD : L.invD, L.pin};
+}
+
+// The dense coarse operators of the hierarchy in the current pressure mode (2D), made
+// once. A context without them (no level small enough, no memory for them, a stream
+// that is being captured when they would be made) solves its coarsest level in CTA 0.
+static int dense_make(fem_ctx* c, cudaStream_t s) {
+  const int pinned = c->set_zeroP;
+  if (c->g.kind == FEM_HEX8 || c->nlev < 2 || c->dense_made[pinned] || !dense_usable(c)) return FEM_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  FEM_CHECK(cudaStreamIsCapturing(s, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return FEM_OK;
   FemDenseLevel lv[FEM_MAX_LEVELS];
-  for (int l = 0; l < c->nlev; ++l) {
-    const CtxLevel& L = c->lv[l];
-    lv[l] = FemDenseLevel{L.g, lattice_of(L.g), L.tab, L.tab_off, c->set_zeroP ? L.winvD : L.invD,
-                          l == 0 ? c->pin0 : L.pin};
-  }
+  for (int l = 0; l < c->nlev; ++l) lv[l] = dense_level_of(c, l);
   FemDense* d = nullptr;
-  const int rc = fem_dense_acquire(&d, lv, c->nlev, c->set_zeroP, c->lx, c->ly, c->device, c->sms, s);
-  if (rc == FEM_E_CUDA && cudaGetLastError() == cudaErrorMemoryAllocation) d = nullptr;
-  else if (rc) return rc;
-  fem_dense_release(c->dense);
-  c->dense = d;
+  const int rc = fem_dense_acquire(&d, lv, c->nlev, pinned, c->lx, c->ly, c->device, c->sms, s);
+  if (rc && !(rc == FEM_E_CUDA && cudaGetLastError() == cudaErrorMemoryAllocation)) return rc;
+  c->dense[pinned] = d;
+  c->dense_made[pinned] = true;
+  // level 0 in pinned mode, where a solve on all CTAs would apply it
+  int ld;
+  const long long n = c->g.nn, ctas = c->g.kind == FEM_Q1_2D ? (n + 511) / 512 : c->coop_capacity;
+  if (pinned && n <= FEM_DENSE_NN && n * n <= ctas * FEM_DENSE_ENTRIES && fem_dense_matrix(d, c->nlev - 2, &ld) &&
+      dalloc(&c->dense0, n * fem_dense_ld((int)n)))
+    cudaGetLastError();  // no memory for it: from level 1
   return FEM_OK;
+}
+
+// The level-0 matrix for the current pins, in place and in stream order
+static int dense_renew(fem_ctx* c, cudaStream_t s) {
+  if (!c->dense0) return FEM_OK;
+  FemDenseLevel lv[2] = {dense_level_of(c, 0), dense_level_of(c, 1)};
+  lv[0].invD = c->lv[0].winvD;
+  int ldc = 0;
+  const double* Cc = fem_dense_matrix(c->dense[1], c->nlev - 2, &ldc);
+  return fem_dense_finest(lv, Cc, ldc, c->dense0, fem_dense_ld(c->g.nn), c->sms, s);
 }
 
 extern "C" int fem_ctx_set_bc(fem_ctx* c, const uint8_t* dmask, const uint8_t* pmask, int set_zeroP,
@@ -635,7 +674,6 @@ extern "C" int fem_ctx_set_bc(fem_ctx* c, const uint8_t* dmask, const uint8_t* p
     FEM_CHECK(cudaMemcpyAsync(c->pmask, pmask, nn, cudaMemcpyDeviceToDevice, s));
     FEM_CHECK(cudaMemcpyAsync(c->aipin, pmask, nn, cudaMemcpyDeviceToDevice, s));
   }
-  const bool mode_changed = c->set_zeroP != (set_zeroP ? 1 : 0);
   c->set_zeroP = set_zeroP ? 1 : 0;
   if (c->mg2) {  // its pins and mean-zero form follow the boundary sets
     FEM_CHECK(cudaStreamSynchronize(s));
@@ -644,8 +682,8 @@ extern "C" int fem_ctx_set_bc(fem_ctx* c, const uint8_t* dmask, const uint8_t* p
   }
   FEM_TRY(fem_launch_invdiag(c->g.nn, c->Ldiag, c->pmask, c->lv[0].invD, c->lv[0].winvD, s));
   c->pin0 = c->pmask;
-  if (c->nlev > 1 && (mode_changed || pmask)) FEM_TRY(dense_refresh(c, s));
-  return FEM_OK;
+  FEM_TRY(dense_make(c, s));
+  return dense_renew(c, s);
 }
 
 extern "C" int fem_ctx_setup_multigrid(fem_ctx* c, int nlev, const uint8_t* level_pmasks, double coarse_tol,
@@ -679,11 +717,10 @@ extern "C" int fem_ctx_setup_multigrid(fem_ctx* c, int nlev, const uint8_t* leve
   }
   mg3_destroy(c->mg2);
   c->mg2 = nullptr;
-  fem_dense_release(c->dense);
-  c->dense = nullptr;
   const FemGrid& g0 = c->g;
   for (int l = 1; l < nlev; ++l)
     if ((g0.nex >> l) < 1 || (g0.ney >> l) < 1) return FEM_E_ARG;
+  dense_drop(c);
   // release previous levels
   for (int l = 1; l < FEM_MAX_LEVELS; ++l) {
     CtxLevel& L = c->lv[l];
@@ -781,7 +818,8 @@ extern "C" int fem_ctx_setup_multigrid(fem_ctx* c, int nlev, const uint8_t* leve
   FEM_ALLOC(c->cp, ncn);
   FEM_ALLOC(c->cq, ncn);
   c->pin0 = c->lv[0].pin;
-  return dense_refresh(c, s);
+  FEM_TRY(dense_make(c, s));
+  return dense_renew(c, s);
 }
 
 extern "C" int fem_ctx_level_info(const fem_ctx* c, int level, int* nn, int* nnx, int* nny, int* nex, int* ney) {

@@ -16,6 +16,10 @@
 // Contexts with the same coarse levels (lattices, box, pins, pressure mode)
 // share one set of matrices: a server's many solvers read one copy from L2. The
 // registry holds weak references only, so a set is freed with its last context.
+// A set depends on nothing that changes under a hierarchy: the pins of level 0
+// follow fem_ctx_set_bc, so a pinned level 0 has no matrix here but one of its
+// context's own, rebuilt in place (fem_dense_finest). Graphs and packs may hold
+// pointers to either for as long as the hierarchy lives.
 #include <cstring>
 #include <map>
 #include <memory>
@@ -250,7 +254,7 @@ int build(DenseStore* D, const FemDenseLevel* lv, int pinned, int sms, cudaStrea
   for (int l = D->nlev - 1; l >= 0; --l) {
     const FemDenseLevel& L = lv[l];
     const int n = L.g.nn;
-    D->ld[l] = (n + 3) & ~3;  // rows start on 32 bytes
+    D->ld[l] = fem_dense_ld(n);
     const size_t bytes = sizeof(double) * (size_t)n * D->ld[l];
     DENSE_CUDA(cudaMalloc(&D->C[l], bytes));
     DENSE_CUDA(cudaMemsetAsync(D->C[l], 0, bytes, s));
@@ -288,7 +292,7 @@ int fem_dense_acquire(FemDense** out, const FemDenseLevel* lv, int nlev, int pin
                       int sms, cudaStream_t s) {
   *out = nullptr;
   int f = nlev;
-  while (f > 0 && lv[f - 1].g.nn <= FEM_DENSE_NN) --f;
+  while (f > (pinned ? 1 : 0) && lv[f - 1].g.nn <= FEM_DENSE_NN) --f;
   if (f == nlev || lv[0].g.kind == FEM_HEX8) return FEM_OK;
   const FemDenseLevel* d = lv + f;
   const int nd = nlev - f;
@@ -332,6 +336,14 @@ int fem_dense_acquire(FemDense** out, const FemDenseLevel* lv, int nlev, int pin
     return FEM_E_OOM;
   }
   return FEM_OK;
+}
+
+int fem_dense_finest(const FemDenseLevel* lv, const double* Cc, int ldc, double* C, int ld, int sms, cudaStream_t s) {
+  const int n = lv[0].g.nn, blocks = fem_nblocks(n, 1, sms * 8);
+  DENSE_CUDA(cudaMemsetAsync(C, 0, sizeof(double) * (size_t)n * ld, s));
+  const DenseArgs A{lv[0], lv[1], Cc, ldc, C, ld};
+  return lv[0].g.kind == FEM_Q1_2D ? launch_level<FEM_Q1_2D, true>(A, blocks, s)
+                                   : launch_level<FEM_Q2_2D, true>(A, blocks, s);
 }
 
 void fem_dense_release(FemDense* d) { delete d; }
