@@ -130,7 +130,7 @@ struct fem_ctx {
   FemDense* dense[2] = {};
   bool dense_made[2] = {};
   double* dense0 = nullptr;
-  const uint8_t* pin0 = nullptr;  // the gamma_p mask that level 0's winvD was made from
+  uint8_t* mpin0 = nullptr;       // the gamma_p mask that level 0's winvD was made from, rewritten in place (2D)
   double *cr = nullptr, *cp = nullptr, *cq = nullptr;  // coarse CG scratch
   // barrier / reduction state
   unsigned int* bar = nullptr;
@@ -362,7 +362,7 @@ extern "C" void fem_ctx_destroy(fem_ctx* c) {
   mixmom_destroy(c->mixmom);
   dense_drop(c);
   void* ptrs[] = {c->coords, c->wq, c->N, c->dN, c->Me, c->Le, c->Leoff, c->Ge, c->M, c->Ldiag, c->Kd,
-                  c->dmask, c->pmask, c->aipin, c->cr, c->cp, c->cq, c->bar, c->err, c->partials, c->pr,
+                  c->dmask, c->pmask, c->aipin, c->mpin0, c->cr, c->cp, c->cq, c->bar, c->err, c->partials, c->pr,
                   c->pz, c->pp0, c->pp1, c->pAp, c->br, c->brh, c->bp0, c->bp1, c->bq0, c->bq1, c->bt,
                   c->rhsU, c->Uhat, c->gPn, c->Ustar, c->rhsP, c->Ce, c->Ce2, c->Ct, c->Mt, c->Ek, c->tau,
                   c->dotpart, c->Fe, c->flags, c->vcv, c->cvf, c->ebe_tab, c->bs_cnt, c->bs_off, c->bs_list, c->vjp, c->vjp2,
@@ -493,6 +493,7 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   FEM_ALLOC(c->dmask, vn + 4);  // whole words
   FEM_ALLOC(c->pmask, nn + 4);  // whole words (fem_ring_copy_mask)
   FEM_ALLOC(c->aipin, nn + 4);
+  if (g.kind != FEM_HEX8) FEM_ALLOC(c->mpin0, nn + 4);
   FEM_ALLOC(c->bar, 1);
   FEM_ALLOC(c->err, 1);
   FEM_ALLOC(c->partials, (size_t)FEM_NSLOTS * max_columns(c));
@@ -681,7 +682,7 @@ extern "C" int fem_ctx_set_bc(fem_ctx* c, const uint8_t* dmask, const uint8_t* p
     c->mg2 = nullptr;
   }
   FEM_TRY(fem_launch_invdiag(c->g.nn, c->Ldiag, c->pmask, c->lv[0].invD, c->lv[0].winvD, s));
-  c->pin0 = c->pmask;
+  if (c->mpin0) FEM_CHECK(cudaMemcpyAsync(c->mpin0, c->pmask, nn, cudaMemcpyDeviceToDevice, s));
   FEM_TRY(dense_make(c, s));
   return dense_renew(c, s);
 }
@@ -817,7 +818,7 @@ extern "C" int fem_ctx_setup_multigrid(fem_ctx* c, int nlev, const uint8_t* leve
   FEM_ALLOC(c->cr, ncn);
   FEM_ALLOC(c->cp, ncn);
   FEM_ALLOC(c->cq, ncn);
-  c->pin0 = c->lv[0].pin;
+  FEM_CHECK(cudaMemcpyAsync(c->mpin0, c->lv[0].pin, c->g.nn, cudaMemcpyDeviceToDevice, s));
   FEM_TRY(dense_make(c, s));
   return dense_renew(c, s);
 }
@@ -963,7 +964,7 @@ static void fill_cg_args(fem_ctx* c, CgArgs& A) {
     M.r = (l == 0) ? c->pr : L.r;
     M.t = L.t;
   }
-  for (int l = 0; l < A.nlev; ++l) A.lv[l].mpin = (l == 0 && c->pin0) ? c->pin0 : A.lv[l].pin;
+  for (int l = 0; l < A.nlev; ++l) A.lv[l].mpin = l == 0 ? c->mpin0 : A.lv[l].pin;
   // level 0 pins of the plain (non-multigrid) solve are the context gamma_p
   if (c->nlev == 1 || !c->lv[0].pin) A.lv[0].pin = c->pmask;
   A.dense_lv = A.nlev;

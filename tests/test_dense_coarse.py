@@ -92,10 +92,11 @@ def test_two_iterations(order, nex, ney, nlev, pinned, periodic, faces):
     assert float(np.linalg.norm(x.cpu().numpy() - xo)) <= 1e-10 * float(np.linalg.norm(xo))
 
 
-@pytest.mark.parametrize("order,nex,ney,nlev", SMALL)
+@pytest.mark.parametrize("order,nex,ney,nlev", SMALL + [(1, 64, 64, 4), (2, 40, 24, 3)])
 def test_captured_solve_follows_set_bc(order, nex, ney, nlev):
     """A captured pinned solve, replayed after the pins changed and after the context went to
-    mean-zero pressure: the bits of a direct pinned solve with the pins of that moment."""
+    mean-zero pressure: the bits of a direct pinned solve with the pins of that moment (the
+    larger lattices read them in their sweeps, not in a matrix)."""
     ctx = _context(order, nex, ney, nlev, True)
     x, call = _solver(ctx, _rhs(ctx.nn))
     call()
