@@ -137,7 +137,8 @@ struct fem_ctx {
   int* err = nullptr;
   double* partials = nullptr;
   int max_coop = 148;       // CTAs of the persistent cooperative launches
-  int coop_capacity = 148;  // upper bound of max_coop (co-resident capacity)
+  int coop_capacity = 148;  // upper bound of max_coop (co-resident capacity, FEM_MAX_CTAS)
+  int device_ctas = 148;    // co-resident capacity of the device
   // vectors (nn or ndim*nn)
   double *pr = nullptr, *pz = nullptr, *pp0 = nullptr, *pp1 = nullptr, *pAp = nullptr;  // CG
   double *br = nullptr, *brh = nullptr, *bp0 = nullptr, *bp1 = nullptr, *bq0 = nullptr, *bq1 = nullptr,
@@ -212,8 +213,28 @@ static int ctx_grid_for(const fem_ctx* c) { return nblocks(c->g.nn, FEM_THREADS,
 // A CG solve whose bits depend on its work items, not its grid (fem_items)
 static bool cg_by_items(const fem_ctx* c) { return c->g.kind == FEM_Q1_2D && c->set_zeroP; }
 
-// CTAs whose matrix share picks the dense level of a solve by items
-static long long dense_ctas(const fem_ctx* c) { return cg_by_items(c) ? ctx_grid_for(c) : c->max_coop; }
+// CTAs that a solve may take without a cap. A solver CTA has an SM to itself and a
+// cooperative launch waits until all its CTAs fit, so a small solve on the whole
+// device would take turns with those of other streams. It takes 1 / n of the device,
+// the largest n that costs it about nothing: `want` in [1, most].
+static int side_ctas(const fem_ctx* c, int want, int most) {
+  return std::min(c->max_coop, c->device_ctas / std::max(1, std::min(want, most)));
+}
+// Solves whose sums are kept per CTA: about two shares of nodes / 512. Under multigrid
+// half the device for the solves of which eight would fit at nodes / 512, and the whole
+// for larger ones: their sums' order decides iteration counts of long runs (64^2 quad9).
+// One stream and eight, on nodes / 512 CTAs -> the whole device -> this rule, us per step:
+// channel on 90 x 33 quad9 6690, 1179 -> 5087, 4855 -> 5143, 1699; 3D box 50 x 21 x 19
+// 3775, 1241 -> 2132, 2060 -> 2164, 1083; 24 x 10 x 10 2102, 294 -> 1139, 430 -> 1122, 180;
+// vortex 64^2 quad4 736, 119 -> 312, 283 -> 320, 152.
+static int node_ctas(const fem_ctx* c, bool mg) {
+  const int share = nblocks(c->g.nn, FEM_THREADS, c->device_ctas);
+  if (mg) return side_ctas(c, 8 * share <= c->device_ctas ? 2 : 1, 2);
+  return side_ctas(c, (c->device_ctas + share) / (2 * share), 6);
+}
+
+// CTAs whose matrix share picks the dense level of a solve
+static long long dense_ctas(const fem_ctx* c) { return cg_by_items(c) ? ctx_grid_for(c) : node_ctas(c, true); }
 
 // The level from which a solve applies the dense coarse operator: the finest whose
 // matrix is at most FEM_DENSE_ENTRIES entries per CTA, where its product costs as
@@ -245,17 +266,27 @@ static int max_columns(const fem_ctx* c) {
   return std::max({c->coop_capacity, c->sms * (FEM_CG_THREADS / 32), strips});
 }
 
-// CTAs of a CG solve: one warp of work per CTA while there are items (a warp
-// alone on its SM runs fastest: 64^2 quad4 cavity step on 9 CTAs 541 us, on 145
-// 373 us), and enough for the dense level's rows.
-static int cg_grid_for(const fem_ctx* c) {
-  if (c->g.kind == FEM_HEX8) return (int)std::min<long long>(c->max_coop, fem_l3_units(c->g));
-  if (cg_by_items(c)) return std::min(cg_items(c), c->max_coop);
+// CTAs of a solve by items: up to three items each, which share an SM at no cost
+// (64^2 quad4 cavity step on 9 CTAs 452 us, on 37 286, on 48 to 148 281).
+static int item_ctas(const fem_ctx* c) {
+  const int items = cg_items(c);
+  return std::min(items, side_ctas(c, 3 * c->device_ctas / items, 3));
+}
+
+// CTAs of a CG solve: ~64 nodes each and enough for the dense level's rows; on part of
+// the device not a multiple of the strips, which gives all warps of a CTA the same strip
+// (90 x 33 quad9, 7 strips: 5148 us on 48 CTAs, 5650 on 49, 5544 on 56, 4997 on 60).
+static int cg_grid_for(const fem_ctx* c, int prec) {
+  if (cg_by_items(c)) return item_ctas(c);
+  int most = node_ctas(c, prec == FEM_PREC_MG);
+  if (c->g.kind == FEM_HEX8) return (int)std::min<long long>(most, fem_l3_units(c->g));
+  const int own = c->g.kind == FEM_Q2_2D ? KS<FEM_Q2_2D>::OWN : KS<FEM_Q1_2D>::OWN, strips = (c->g.nnx + own - 1) / own;
+  if (most < c->max_coop && strips > 1 && most % strips == 0) --most;
   const double* C;
   int ld;
   const int d = dense_level(c, &C, &ld);
   const long long n = d < c->nlev ? c->lv[d].g.nn : 0;
-  return std::max(nblocks(c->g.nn, 64, c->max_coop), nblocks((n + 7) / 8, 1, c->max_coop));
+  return std::max(nblocks(c->g.nn, 64, most), nblocks((n + 7) / 8, 1, most));
 }
 
 // --------------------------------------------------------------- mesh ----
@@ -467,7 +498,7 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   int occ_cg = 0, occ_bi = 0;
   if (fem_coop_occupancy_cg(&occ_cg) || fem_coop_occupancy_bi(&occ_bi)) return set_err("occupancy", cudaGetLastError());
   const int occ = std::max(1, std::min(occ_cg, occ_bi));
-  c->max_coop = c->sms * occ;
+  c->max_coop = c->device_ctas = c->sms * occ;
   const char* ev = getenv("FEM_MAX_CTAS");
   if (ev && atoi(ev) > 0) c->max_coop = std::min(c->max_coop, atoi(ev));
   c->coop_capacity = c->max_coop;
@@ -974,7 +1005,7 @@ static void fill_cg_args(fem_ctx* c, CgArgs& A) {
 static void set_cg_plan(const fem_ctx* c, CgArgs& A) {
   if (c->g.kind == FEM_HEX8) return;
   const bool by_items = cg_by_items(c);
-  const int grid = cg_grid_for(c), items = by_items ? cg_items(c) : grid * (FEM_CG_THREADS / 32);
+  const int grid = cg_grid_for(c, A.prec), items = by_items ? cg_items(c) : grid * (FEM_CG_THREADS / 32);
   int cols = items;  // of a solve by items: as many as the largest plan has items
   for (int l = 0; l < A.nlev; ++l) {
     MgLevel& M = A.lv[l];
@@ -1014,7 +1045,7 @@ static int run_cg(fem_ctx* c, const double* b, double* x, double tol, double ato
   A.status = status;
   A.final_rr = nullptr;
   FEM_TRY(reset_sync(c, s));
-  const int grid = cg_grid_for(c);
+  const int grid = cg_grid_for(c, precond);
   A.sync.ncols = grid;
   set_cg_plan(c, A);
   double* cr = c->cr ? c->cr : c->pz;
@@ -1093,9 +1124,10 @@ extern "C" int fem_mg_vcycle(fem_ctx* c, const double* r, double* z, cudaStream_
   fill_cg_args(c, A);
   FEM_CHECK(cudaMemcpyAsync(c->pr, r, sizeof(double) * c->g.nn, cudaMemcpyDeviceToDevice, s));
   FEM_TRY(reset_sync(c, s));
+  A.prec = FEM_PREC_MG;
   set_cg_plan(c, A);
   A.dense_lv = A.nlev;  // the reference's coarsest solve
-  return fem_launch_vcycle(A, cg_grid_for(c), c->cr, c->cp, c->cq, z, s);
+  return fem_launch_vcycle(A, cg_grid_for(c, A.prec), c->cr, c->cp, c->cq, z, s);
 }
 
 // Items of the quad4 momentum solve, as many as the CG's, and the columns of its sums
@@ -1142,9 +1174,9 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
   // the hex8 march splits to single planes, the quad4 one to its items
   int grid = ctx_grid_for(c), threads = FEM_THREADS;
   if (c3) {
-    grid = (int)std::min<long long>(c->max_coop, fem_c3_units(c->g));
+    grid = (int)std::min<long long>(node_ctas(c, false), fem_c3_units(c->g));
   } else if (c2) {
-    grid = std::min(cg_items(c), c->max_coop);
+    grid = item_ctas(c);
   } else if (!cvf && c->g.kind != FEM_HEX8) {
     // explicit element matrices, tiles of 32 columns and a row per warp: where tiles of
     // 16 rows leave CTAs idle, 8 rows and a tile per CTA
