@@ -533,7 +533,6 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
   for (double** p : {&c->br, &c->brh, &c->bp0, &c->bp1, &c->bq0, &c->bq1, &c->bt, &c->rhsU, &c->Uhat, &c->gPn,
                      &c->Ustar})
     FEM_ALLOC(*p, vn);
-  FEM_ALLOC(c->Ce, (size_t)g.ne * per);
   FEM_ALLOC(c->vcv, vn);
   FEM_ALLOC(c->ebe_tab, FEM_TAB_MAX);
   if (g.kind != FEM_HEX8) FEM_ALLOC(c->cvf, (size_t)3 * c->nq * g.ne);
@@ -603,6 +602,8 @@ static int ctx_create_impl(const fem_mesh_desc* m, int device, fem_ctx* c) {
     // that does not factor) fem_step4 builds Ce explicitly
     if (g.kind == FEM_Q2_2D && !q2_tensor_factors(c->qt)) c->conv_otf = 0;
   }
+  // hex8 on the fly: 512 bytes per element that only the scalar's matrices would use (transport_mats)
+  if (g.kind != FEM_HEX8 || !c->conv_otf) FEM_ALLOC(c->Ce, (size_t)g.ne * per);
   return FEM_OK;
 }
 
@@ -1347,13 +1348,9 @@ static int transport_mats(fem_ctx* c, const double* Un, const double* U, double 
                           cudaStream_t s) {
   const FemGrid& g = c->g;
   const size_t per = (size_t)g.nen * g.nen, ntot = (size_t)g.ne * per;
-  if (!c->Ce2) {
-    FEM_ALLOC(c->Ce2, ntot);
-    FEM_ALLOC(c->Ct, ntot);
-    FEM_ALLOC(c->Mt, ntot);
-    FEM_ALLOC(c->Ek, ntot);
-    FEM_ALLOC(c->tau, g.ne);
-  }
+  for (double** p : {&c->Ce, &c->Ce2, &c->Ct, &c->Mt, &c->Ek})
+    if (!*p) FEM_ALLOC(*p, ntot);
+  if (!c->tau) FEM_ALLOC(c->tau, g.ne);
   const FemQuad Q = quad_of(c);
   // Ce(U_n, 1) -> Ce, Ce(U, 1) -> Ce2 (solvers/passive_transport.py:80-81)
   FEM_TRY(fem_launch_convection(g, Q, Un, 1.0, 0, c->Ce, s));
