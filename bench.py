@@ -116,7 +116,7 @@ class ClockSampler:
         return {"sm_mhz": statistics.median(load), "sm_max_mhz": mx, "reasons": reasons, "samples": len(rows)}
 
 
-def cg_algorithmic_bytes(level_nn, iters, block_from):
+def cg_algorithmic_bytes(level_nn, iters):
     """Algorithmic DRAM bytes of one k_cg launch (MG-PCG, mean-zero). Per phase:
     the nn-length vectors it must read and write once (FP64), stencil re-reads
     excluded. Init: b, x0 -> r: 3 nn. Per iteration: the direction phase reads z,
@@ -231,7 +231,7 @@ def run_ours(args, rank, world, local_rank):
     d2h = h2d
     res = dict(total_ms=total_ms, step_ms=step_ms, stage_ms=(stage_ms / args.steps).tolist(), iters=iters,
                launches=launches, clocks=clk.summary(), e2e_ms=e2e_ms, h2d=h2d, d2h=d2h, nn=nn, ctx=ctx,
-               level_nn=[ctx.level_info(l)[0] for l in range(ctx.nlev)], block_from=None,
+               level_nn=[ctx.level_info(l)[0] for l in range(ctx.nlev)],
                final=(U.clone(), P.clone()), coords=nc)
     return res
 
@@ -406,7 +406,7 @@ def poisson(n, solves=5):
     iters = int(it.item())
     status = int(stt.item())
     x64 = x.clone()
-    byts = cg_algorithmic_bytes([ctx.level_info(l)[0] for l in range(ctx.nlev)], iters, None)
+    byts = cg_algorithmic_bytes([ctx.level_info(l)[0] for l in range(ctx.nlev)], iters)
     # reference solution for the error figures: FP64 MG-PCG to 1e-12 (untimed)
     xr = torch.zeros_like(b)
     _lib.call("fem_pressure_solve", ctx.handle, ptr(b), ptr(xr), 1e-12, 0.0, 1000, 4, 0, 1, ptr(it), ptr(stt),
@@ -963,7 +963,7 @@ def main():
     share = {k: v / stage_tot for k, v in stage.items()} if stage_tot > 0 else {}
     p_iters = [pi for _, pi in r["iters"]]
     u_iters = [ui for ui, _ in r["iters"]]
-    cg_bytes = np.mean([cg_algorithmic_bytes(r["level_nn"], it, None) for it in p_iters])
+    cg_bytes = np.mean([cg_algorithmic_bytes(r["level_nn"], it) for it in p_iters])
     cg_ms = stage["pressure_pcg"]
     traffic = None
     tp = os.path.join(ROOT, "profiles", "k_cg_tg256_traffic.json")

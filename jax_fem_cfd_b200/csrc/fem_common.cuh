@@ -19,7 +19,6 @@
 #define FEM_Q2_2D 1
 #define FEM_HEX8 2
 
-#define FEM_MAX_NEN 9
 
 struct FemGrid {
   int kind;       // FEM_Q1_2D | FEM_Q2_2D | FEM_HEX8
@@ -58,11 +57,6 @@ __device__ __forceinline__ int fem_local_index(int kind, int di, int dj, int dk)
   if (kind == FEM_Q2_2D) return (int)((FEM_Q2_INV >> (4 * (dj * 3 + di))) & 15ull);
   return (int)((FEM_Q1_INV >> (2 * (dj * 2 + di))) & 3u) + 4 * dk;
 }
-
-struct FemElem {
-  int ie, je, ke;
-  int e;
-};
 
 __device__ __forceinline__ int fem_node_at(const FemGrid& g, int i, int j, int k) {
   if (g.periodic) {
@@ -185,9 +179,6 @@ __device__ __forceinline__ unsigned int fem_ld_acquire(const unsigned int* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void fem_st_release(unsigned int* p, unsigned int v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ unsigned long long fem_globaltimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -255,7 +246,6 @@ __device__ __forceinline__ void fem_stage_wait() {
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
 }
-__device__ __forceinline__ int fem_floordiv2(int v) { return v >> 1; }  // arithmetic shift: floor for v < 0
 // v mod n in [0, n) for any int v (periodic lattice coordinates of staged halos,
 // which can lie more than one period away when a tile is wider than the level)
 __device__ __forceinline__ int fem_wrap(int v, int n) {
@@ -451,16 +441,6 @@ struct GridReducer {
     if constexpr (ITEMS) return tm.sync();
     return tm.template reduce_sync<K>(v, slots, smem);
   }
-  // One block sum for K values bound for any K slots.
-  template <int K>
-  __device__ __forceinline__ void reduce_slots(double (&v)[K], const int (&slots)[K], double* smem) const {
-    fem_block_sum<K>(v, smem);
-    if (threadIdx.x == 0) {
-      double* part = s->partials;
-#pragma unroll
-      for (int q = 0; q < K; ++q) part[(size_t)slots[q] * s->ncols + blockIdx.x] = v[q];
-    }
-  }
   // Totals of K <= 8 slots (any slot numbers). Thread c loads column c (and every
   // data_warps() * 32th after it) of every slot (all loads of a thread in flight at
   // once), warps combine theirs by a fixed shuffle tree, and every thread adds the
@@ -533,51 +513,3 @@ struct GridReducer {
     result_slots<K>(out, sl, smem);
   }
 };
-
-struct BlockReducer {
-  double* store;  // shared memory, >= nslots doubles
-  template <int K>
-  __device__ __forceinline__ void reduce(double (&v)[K], int slot, double* smem) const {
-    fem_block_sum<K>(v, smem);
-    if (threadIdx.x == 0)
-#pragma unroll
-      for (int q = 0; q < K; ++q) store[slot + q] = v[q];
-  }
-  template <int K>
-  __device__ __forceinline__ void reduce_slots(double (&v)[K], const int (&slots)[K], double* smem) const {
-    fem_block_sum<K>(v, smem);
-    if (threadIdx.x == 0)
-#pragma unroll
-      for (int q = 0; q < K; ++q) store[slots[q]] = v[q];
-  }
-  template <int K>
-  __device__ __forceinline__ void result_slots(double (&out)[K], const int (&slots)[K], double*) const {
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < K; ++q) out[q] = store[slots[q]];
-  }
-  template <int K>
-  __device__ __forceinline__ void result(double (&out)[K], int slot, double*) const {
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < K; ++q) out[q] = store[slot + q];
-  }
-};
-
-__device__ __forceinline__ bool fem_isfinite(double x) { return isfinite(x); }
-
-// Node iteration in 2D tiles of 32 x (blockDim/32) lattice nodes, one tile per
-// CTA at a time, so stencil neighbours in adjacent rows are read by the same
-// CTA (L1 hits). f(n, x, y, z) with n the node index of lattice (x, y, z).
-template <class Team, class F>
-__device__ __forceinline__ void fem_tile_loop(const Team& tm, int nx, int ny, int nz, F&& f) {
-  const int TY = blockDim.x >> 5;
-  const int ntx = (nx + 31) >> 5, nty = (ny + TY - 1) / TY;
-  const int nt2 = ntx * nty, ntile = nt2 * nz;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int t = tm.cta(); t < ntile; t += tm.ncta()) {
-    const int z = t / nt2, r = t - z * nt2, by = r / ntx, bx = r - by * ntx;
-    const int x = bx * 32 + tx, y = by * TY + ty;
-    if (x < nx && y < ny) f((z * ny + y) * nx + x, x, y, z);
-  }
-}

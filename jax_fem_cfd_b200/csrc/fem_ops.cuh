@@ -13,10 +13,6 @@ struct MatShared {
   double alpha;
   __device__ __forceinline__ double operator()(int, int a, int b, int nen) const { return alpha * A[a * nen + b]; }
 };
-struct MatSharedT {  // transpose of a shared matrix (divergence: Ge_i^T)
-  const double* A;
-  __device__ __forceinline__ double operator()(int, int a, int b, int nen) const { return A[b * nen + a]; }
-};
 // alpha*A + beta*B_e (+ gamma*C_e), B_e / C_e per element, optionally transposed.
 struct MatCombo {
   const double* A;
@@ -37,93 +33,6 @@ struct MatCombo {
     return v;
   }
 };
-
-// y_c[n] for NC components sharing one coefficient provider (x_c = x + c*stride).
-template <int NC, class Mat>
-__device__ __forceinline__ void fem_gather(const FemGrid& g, int n, const Mat& m, const double* __restrict__ x,
-                                           int stride, double (&y)[NC]) {
-#pragma unroll
-  for (int c = 0; c < NC; ++c) y[c] = 0.0;
-  const int nen = g.nen;
-  fem_for_incident(g, n, [&](int ie, int je, int ke, int e, int a) {
-    double part[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) part[c] = 0.0;
-    for (int b = 0; b < nen; ++b) {
-      const double coef = m(e, a, b, nen);
-      const int j = fem_elem_node(g, ie, je, ke, b);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) part[c] += coef * x[j + (size_t)c * stride];
-    }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) y[c] += part[c];
-  });
-}
-
-// Same as fem_gather, but the input value at node j is produced by a functor
-// (used to fuse a pointwise producer into the stencil: x_j = f(j)).
-template <class Mat, class Src>
-__device__ __forceinline__ double fem_gather_fn(const FemGrid& g, int n, const Mat& m, const Src& src) {
-  double y = 0.0;
-  const int nen = g.nen;
-  fem_for_incident(g, n, [&](int ie, int je, int ke, int e, int a) {
-    double part = 0.0;
-    for (int b = 0; b < nen; ++b) {
-      const int j = fem_elem_node(g, ie, je, ke, b);
-      part += m(e, a, b, nen) * src(j);
-    }
-    y += part;
-  });
-  return y;
-}
-
-// Gradient: y_d[n] = sum Ge_d rows * P (ND outputs from one input).
-template <int ND>
-__device__ __forceinline__ void fem_gather_grad(const FemGrid& g, int n, const double* Ge, const double* __restrict__ P,
-                                                double (&y)[ND]) {
-#pragma unroll
-  for (int d = 0; d < ND; ++d) y[d] = 0.0;
-  const int nen = g.nen, nen2 = nen * nen;
-  fem_for_incident(g, n, [&](int ie, int je, int ke, int e, int a) {
-    double part[ND];
-#pragma unroll
-    for (int d = 0; d < ND; ++d) part[d] = 0.0;
-    for (int b = 0; b < nen; ++b) {
-      const double pj = P[fem_elem_node(g, ie, je, ke, b)];
-#pragma unroll
-      for (int d = 0; d < ND; ++d) part[d] += Ge[d * nen2 + a * nen + b] * pj;
-    }
-#pragma unroll
-    for (int d = 0; d < ND; ++d) y[d] += part[d];
-  });
-}
-
-// Divergence: y[n] = sum_d sum Ge_d^T rows * U_d (reference sums the per-component
-// assembled vectors, core/element_mult.py:147-155).
-template <int ND>
-__device__ __forceinline__ double fem_gather_div(const FemGrid& g, int n, const double* Ge, const double* __restrict__ U,
-                                                 int nn) {
-  double acc[ND];
-#pragma unroll
-  for (int d = 0; d < ND; ++d) acc[d] = 0.0;
-  const int nen = g.nen, nen2 = nen * nen;
-  fem_for_incident(g, n, [&](int ie, int je, int ke, int e, int a) {
-    double part[ND];
-#pragma unroll
-    for (int d = 0; d < ND; ++d) part[d] = 0.0;
-    for (int b = 0; b < nen; ++b) {
-      const int j = fem_elem_node(g, ie, je, ke, b);
-#pragma unroll
-      for (int d = 0; d < ND; ++d) part[d] += Ge[d * nen2 + b * nen + a] * U[j + (size_t)d * nn];
-    }
-#pragma unroll
-    for (int d = 0; d < ND; ++d) acc[d] += part[d];
-  });
-  double y = acc[0];
-#pragma unroll
-  for (int d = 1; d < ND; ++d) y += acc[d];
-  return y;
-}
 
 // ---------------------------------------------------------------------------
 // Element matrices from quadrature data (core/element_calc.py:165-200).

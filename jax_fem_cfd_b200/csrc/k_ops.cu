@@ -232,19 +232,6 @@ __global__ void k_supg_tau(FemGrid g, FemQuad Q, const double* __restrict__ U, c
   }
 }
 
-// Combined per-element matrix for the SUPG scalar operator:
-// out_e = s_m * tau_e * Cn_e^T + s_c * (C_e + tau_e * Ct_e)   (transport lhs/rhs).
-__global__ void k_supg_combine(int ne, int nen, const double* __restrict__ tau, const double* __restrict__ Cn,
-                               const double* __restrict__ C, const double* __restrict__ Ct, double s_m, double s_c,
-                               double* __restrict__ out) {
-  const int per = nen * nen;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)ne * per; t += gridDim.x * blockDim.x) {
-    const size_t e = t / per;
-    const int ab = (int)(t % per), a = ab / nen, b = ab % nen;
-    out[t] = s_m * (tau[e] * Cn[e * per + b * nen + a]) + s_c * (C[t] + tau[e] * Ct[t]);
-  }
-}
-
 // ------------------------------------------------------------- transfers ----
 __global__ void k_interp(FemLattice H, FemLattice h, const double* __restrict__ xH, double* __restrict__ xh) {
   const int ux = h.ux(), n = ux * h.uy();
