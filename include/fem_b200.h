@@ -365,9 +365,12 @@ int fem_ctx_set_trace(fem_ctx* ctx, unsigned long long* buf, int cap);
  * (optional) receives that capacity (SMs x resident solver CTAs per SM). A
  * request loop that runs several contexts at once on separate streams gives
  * each a share of the capacity, so every cooperative grid in flight fits on
- * the device at the same time. Results depend on the cap (the reduction
- * partials are per CTA) and are reproducible for a given cap. No reference
- * counterpart: the reference runs one problem at a time. */
+ * the device at the same time. Without a cap a solve takes what a lone one runs
+ * fastest on: part of the device where that costs it about nothing. Results are
+ * reproducible for a given cap and depend on it, as the reduction partials are
+ * per CTA; those of the wall-bounded quad4 pressure solve and the quad4 momentum
+ * solve are per work item, and the same for every cap of nodes / 512 CTAs or
+ * more. No reference counterpart: the reference runs one problem at a time. */
 int fem_ctx_set_max_ctas(fem_ctx* ctx, int ctas, int* capacity);
 
 /* nsteps (even, >= 2) consecutive fem_step4 calls captured into one CUDA

@@ -1,7 +1,7 @@
 // hex8 momentum operator from the nodal velocities: for 3 components
 //   y = (mass Me + diff Le + cc Ce(U)) x,
-// Ce of core/element_calc.py:165-185, beta (div u) on its diagonal term, with no
-// per-element matrix or factor in memory.
+// Ce of core/element_calc.py:165-185, beta (div u) on its diagonal term, from no
+// per-element matrix or factor.
 //
 // The mesh is a lattice of equal boxes, so every interpolation to the 2 x 2 x 2
 // Gauss points factors into three 1D ones, and a derivative is the difference

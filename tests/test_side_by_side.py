@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
                                                             (2, False, 50, 21, 19, 1), (2, False, 9, 9, 9, 1)])
 def test_two_streams_overlap(kind, periodic, nex, ney, nez, nlev):
     """Barrier times of two pressure solves of 200 iterations (milliseconds each; the second
-    is launched some tens of microseconds after the first): they overlap."""
+    is launched some tens of microseconds after the first, in one of three tries): they
+    overlap."""
     from jax_fem_cfd_b200 import _lib
     from jax_fem_cfd_b200.context import Context, Mesh, make_mask, ptr
     from jax_fem_cfd_b200.core import multigrid as mg
@@ -39,16 +40,17 @@ def test_two_streams_overlap(kind, periodic, nex, ney, nez, nlev):
         torch.cuda.synchronize()
 
     run()
-    for ctx, _, _, _, tr, _ in solves:
-        _lib.call("fem_ctx_set_trace", ctx.handle, ptr(tr), cap)
-    torch.cuda.synchronize()
-    run()
+    for s in solves:
+        _lib.call("fem_ctx_set_trace", s[0].handle, ptr(s[4]), cap)
     spans = []
-    for ctx, _, _, it, tr, _ in solves:
-        _lib.call("fem_ctx_set_trace", ctx.handle, None, 0)
-        t = tr.cpu().numpy()
-        t = t[1:int(t[0]) + 1] & ((1 << 56) - 1)
-        spans.append((t.min(), t.max()))
-    (a0, a1), (b0, b1) = spans
-    assert a1 - a0 > 200_000, spans  # ns: long beside the launches
-    assert max(a0, b0) < min(a1, b1), spans
+    for _ in range(3):
+        for s in solves:
+            s[4].zero_()
+        run()
+        t = [s[4].cpu().numpy() for s in solves]
+        t = [v[1:int(v[0]) + 1] & ((1 << 56) - 1) for v in t]
+        spans.append([(int(v.min()), int(v.max())) for v in t])
+    for s in solves:
+        _lib.call("fem_ctx_set_trace", s[0].handle, None, 0)
+    assert all(a1 - a0 > 200_000 for (a0, a1), _ in spans), spans  # ns: long beside the launches
+    assert any(max(a0, b0) < min(a1, b1) for (a0, a1), (b0, b1) in spans), spans
