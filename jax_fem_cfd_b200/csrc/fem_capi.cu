@@ -225,7 +225,7 @@ static int side_ctas(const fem_ctx* c, int want, int most) {
 // for larger ones: their sums' order decides iteration counts of long runs (64^2 quad9).
 // One stream and eight, on nodes / 512 CTAs -> the whole device -> this rule, us per step:
 // channel on 90 x 33 quad9 6690, 1179 -> 5087, 4855 -> 5143, 1699; 3D box 50 x 21 x 19
-// 3775, 1241 -> 2132, 2060 -> 2164, 1083; 24 x 10 x 10 2102, 294 -> 1139, 430 -> 1122, 180;
+// 3775, 1241 -> 2142, 2065 -> 2124, 1380; 24 x 10 x 10 2102, 294 -> 1139, 430 -> 1122, 180;
 // vortex 64^2 quad4 736, 119 -> 312, 283 -> 320, 152.
 static int node_ctas(const fem_ctx* c, bool mg) {
   const int share = nblocks(c->g.nn, FEM_THREADS, c->device_ctas);
@@ -1172,10 +1172,12 @@ static int run_bicgstab(fem_ctx* c, int ncomp, const MatCombo& op, const uint8_t
     A.c2plan = bi_plan(c);
   }
   FEM_TRY(reset_sync(c, s));
-  // the hex8 march splits to single planes, the quad4 one to its items
+  // the hex8 march splits to single planes, the quad4 one to its items. On part of the device
+  // two planes of a CTA would take half as long again: step of the 50 x 21 x 19 box 2124 us on
+  // 80 CTAs here, 2168 on 74 (eight streams 1380 and 1084).
   int grid = ctx_grid_for(c), threads = FEM_THREADS;
   if (c3) {
-    grid = (int)std::min<long long>(node_ctas(c, false), fem_c3_units(c->g));
+    grid = (int)std::min<long long>(c->max_coop, fem_c3_units(c->g));
   } else if (c2) {
     grid = item_ctas(c);
   } else if (!cvf && c->g.kind != FEM_HEX8) {
