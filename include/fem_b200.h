@@ -112,7 +112,7 @@ int fem_ctx_element_data(const fem_ctx* ctx, double* wq, double* N, double* Nder
  * nodes, or node 0 when there is no outlet: setup/simulation.py:178-181).
  * set_zeroP selects pinned (1) or mean-zero (0) pressure (StandardSolverConfig).
  * The sets are rewritten in place: a captured step or a pack made before keeps
- * its pressure mode and reads the new ones. */
+ * its pressure mode and reads the new ones (a Dirichlet set only if it had one). */
 int fem_ctx_set_bc(fem_ctx* ctx, const uint8_t* dmask, const uint8_t* pmask, int set_zeroP, cudaStream_t stream);
 
 /* Multigrid hierarchy (core/multigrid.py:9-88): nlev levels obtained by halving
